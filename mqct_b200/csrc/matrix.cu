@@ -24,6 +24,7 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "finalize.cuh"
 #include "matrix_plan.cuh"
 #include "pes.cuh"
 
@@ -396,150 +397,106 @@ contract_fp64_kernel(int n_rows, int G2, int nR, const int* __restrict__ row_a,
 }
 
 // ------------------------------------------------------------------ K4: finalize
-// finalize_kernel: one CTA per reference element k.
-//  (a) sum the contraction partials of its GEMM row in FP64 (fixed order),
-//      convert to Hartree (times the exact per-column factor of the F16x3
-//      scaling), write Mat_el(:,k) coalesced along R;
-//  (b) MIJ_CUTOFF at R~r_cut1/r_cut2 (MQCT_SOURCE_CODES/matrix_ini.f:1969-1997):
-//      the column is zeroed and flagged when max(|M(ir1)|, |M(ir2)|) < cut;
-//  (c) the clamped cubic spline with finite-difference end slopes
-//      (MQCT_SOURCE_CODES/matrix_ini.f:2005-2016; recurrence of
-//      MQCT_SOURCE_CODES/suppl_routines.f:914-965).  With both end slopes equal
-//      to the end differences, u_0 = 0 and u_n = 0; the remaining recurrence
-//      u_i = t_i - s_i u_{i-1}, y2_i = f_i y2_{i+1} + u_i has grid-only s_i, f_i
-//      and data terms t_i = c_i (d_i - d_{i-1}), d_i = (y_{i+1} - y_i) / h_i,
-//      which all threads form in parallel; one warp evaluates the two first-order
-//      recurrences as scans of affine maps (segments per lane + shuffle scan).
-// Grid coefficients (5 x nR, see MatrixPlan::init): 1/h_i, c_i, s_i, f_i, and
-// in slot [4 nR] the factor of y2_{n-1} = -u_{n-2} / (2 (f_{n-2}/2 + 1)).
-template <class TP>
-__global__ void __launch_bounds__(128)
-finalize_kernel(int64_t P, int nR, const int* __restrict__ k_to_row, const TP* __restrict__ part,
-                int n_part, int64_t part_stride, int ldp, double scale,
-                const double* __restrict__ col_scale, int ir1, int ir2, double cut,
-                const double* __restrict__ gc, double* __restrict__ mat,
-                int* __restrict__ skipped, double* __restrict__ y2) {
+// finalize_kernel: the contraction's partial sums of each element added in FP64 (fixed
+// order), converted to Hartree, then the cut-off and the spline (finalize.cuh), one warp
+// per element; the warps of a persistent grid take elements in turn, so that the grid
+// coefficients and scan multipliers are formed once per warp.
+// One column of partial sums is copied to shared memory (cp.async) while the column before it
+// is worked on: the kernel is bound by those reads and the output, and eight warps of a CTA
+// with a column in flight each keep enough bytes on the way.
+__device__ __forceinline__ void cp_async8(double* dst, const double* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
+                   (uint32_t)__cvta_generic_to_shared(dst)),
+               "l"(src)
+               : "memory");
+}
+template <int LM, int NC>
+__global__ void __launch_bounds__(256, LM == 0 || LM == 17 ? 1 : 2)
+finalize_kernel(int64_t P, FinGrid g, const int* __restrict__ k_to_row,
+                const double* __restrict__ part, int n_part, int64_t part_stride, int ldp,
+                double scale) {
   extern __shared__ double fin_sm[];
-  double* __restrict__ col = fin_sm;           // nR values
-  double* __restrict__ t = fin_sm + nR;        // nR recurrence terms, then u
-  __shared__ double cut_vals[2];
-  const int64_t k = blockIdx.x;
-  const int row = k_to_row[k];
-  if (sizeof(TP) == 4 && (ldp & 3) == 0 && (part_stride & 3) == 0) {
-    // FP32 partials: 16-byte loads, four radial points per thread
-    const float4* src = reinterpret_cast<const float4*>(part) + (size_t)row * (ldp >> 2);
-    for (int i4 = threadIdx.x; 4 * i4 < nR; i4 += blockDim.x) {
-      double v0 = 0.0, v1 = 0.0, v2 = 0.0, v3 = 0.0;
-#pragma unroll 4
-      for (int p = 0; p < n_part; ++p) {
-        const float4 f = __ldg(src + (size_t)p * (part_stride >> 2) + i4);
-        v0 += (double)f.x;
-        v1 += (double)f.y;
-        v2 += (double)f.z;
-        v3 += (double)f.w;
-      }
-      const double vv[4] = {v0, v1, v2, v3};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int i = 4 * i4 + e;
-        if (i < nR) col[i] = vv[e] * (col_scale ? scale * col_scale[i] : scale);
-      }
-    }
-  } else {
-    for (int i = threadIdx.x; i < nR; i += blockDim.x) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int nR = g.nR, ld = fin_len(nR);
+  const int rows = 1 + (LM ? 0 : 1) + n_part;  // shared rows of a warp
+  double* col = fin_sm + kFinMul + (size_t)ld * (4 + warp * rows);
+  double* tb = col + ld;
+  double* stage = col + (size_t)ld * (LM ? 1 : 2);
+  const int64_t step = (int64_t)gridDim.x * nw;
+  // (few columns: every SM gets some, and the idle warps share the set-up)
+  int64_t k0 = (int64_t)warp * gridDim.x + blockIdx.x;
+  int row = k0 < P ? k_to_row[k0] : 0;
+  auto fetch = [&]() {
+    const double* src = part + (size_t)row * ldp;
+    for (int p = 0; p < n_part; ++p, src += part_stride)
+      for (int i = lane; i < nR; i += 32) cp_async8(stage + p * ld + i, src + i);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  if (k0 < P) fetch();
+  FinLane<LM> f;
+  fin_init<LM>(g, fin_sm, f);
+  const double* coef = fin_sm + kFinMul;
+  for (; k0 < P; k0 += step) {
+    const bool more = k0 + step < P;
+    if (more) row = k_to_row[k0 + step];
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncwarp();                      // the copies of every lane are visible
+    for (int i = lane; i < nR; i += 32) {
       double v = 0.0;
-      for (int p = 0; p < n_part; ++p) v += (double)part[(size_t)p * part_stride + (size_t)row * ldp + i];
-      col[i] = v * (col_scale ? scale * col_scale[i] : scale);
+      for (int p = 0; p < n_part; ++p) v += stage[p * ld + i];
+      col[i] = v * scale;
     }
+    __syncwarp();                      // the stage is read, the column complete
+    if (more) fetch();
+    const int64_t k[1] = {k0};
+    fin_columns<LM, NC, 1>(g, f, coef, col, tb, k);
+    __syncwarp();                      // the column is written out
   }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    cut_vals[0] = col[ir1];
-    cut_vals[1] = col[ir2];
-  }
-  __syncthreads();
-  const bool drop = fmax(fabs(cut_vals[0]), fabs(cut_vals[1])) < cut;
-  double* out = mat + (size_t)k * nR;
-  for (int i = threadIdx.x; i < nR; i += blockDim.x) out[i] = drop ? 0.0 : col[i];
-  if (threadIdx.x == 0 && skipped) skipped[k] = drop ? 1 : 0;
-  if (!y2) return;
-  double* oy = y2 + (size_t)k * nR;
-  if (drop || nR < 3) {
-    for (int i = threadIdx.x; i < nR; i += blockDim.x) oy[i] = 0.0;
-    return;
-  }
-  const double* invh = gc;
-  const double* cfac = gc + nR;
-  const double* sfac = gc + 2 * nR;
-  const double* ffac = gc + 3 * nR;
-  for (int i = 1 + threadIdx.x; i < nR - 1; i += blockDim.x) {
-    const double d1 = (col[i + 1] - col[i]) * invh[i];
-    const double d0 = (col[i] - col[i - 1]) * invh[i - 1];
-    t[i] = cfac[i] * (d1 - d0);
-  }
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    // Both recurrences are compositions of affine maps x -> a x + b, evaluated by
-    // one warp: each lane composes the maps of a contiguous segment, a shuffle
-    // scan composes the segments, and each lane replays its segment from the
-    // value entering it.
-    const unsigned full = 0xffffffffu;
-    const int lane = threadIdx.x;
-    const int m = nR - 2;               // interior points 1 .. nR-2
-    const int L = (m + 31) / 32;
-    auto scan = [&](double& al, double& be) {  // exclusive prefix over lanes
-      for (int o = 1; o < 32; o <<= 1) {
-        const double pa = __shfl_up_sync(full, al, o), pb = __shfl_up_sync(full, be, o);
-        if (lane >= o) {
-          be = al * pb + be;
-          al = al * pa;
-        }
-      }
-      const double pa = __shfl_up_sync(full, al, 1), pb = __shfl_up_sync(full, be, 1);
-      al = lane ? pa : 1.0;
-      be = lane ? pb : 0.0;
-    };
-    // forward: u_i = t_i - s_i u_{i-1}, u_0 = 0
-    const int i0 = 1 + lane * L, i1 = min(1 + (lane + 1) * L, nR - 1);
-    double al = 1.0, be = 0.0;
-    for (int i = i0; i < i1; ++i) {
-      const double a = -sfac[i];
-      be = fma(a, be, t[i]);
-      al *= a;
-    }
-    scan(al, be);
-    double u = be;  // the prefix applied to u_0 = 0
-    for (int i = i0; i < i1; ++i) {
-      u = fma(-sfac[i], u, t[i]);
-      t[i] = u;
-    }
-    __syncwarp();
-    const double ylast = gc[4 * nR] * t[nR - 2];  // y2_{n-1}
-    // backward: y2_i = f_i y2_{i+1} + u_i for i = n-2 .. 1 (k = n-2-i ascending)
-    const int k0 = lane * L, k1 = min((lane + 1) * L, m);
-    al = 1.0;
-    be = 0.0;
-    for (int k = k0; k < k1; ++k) {
-      const int i = nR - 2 - k;
-      const double f = ffac[i];
-      be = fma(f, be, t[i]);
-      al *= f;
-    }
-    scan(al, be);
-    double yv = fma(al, ylast, be);
-    for (int k = k0; k < k1; ++k) {
-      const int i = nR - 2 - k;
-      yv = fma(ffac[i], yv, t[i]);
-      col[i] = yv;
-    }
-    __syncwarp();
-    if (lane == 0) {
-      col[nR - 1] = ylast;
-      col[0] = ffac[0] * col[1];  // u_0 = 0
-    }
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < nR; i += blockDim.x) oy[i] = col[i];
+}
+
+// Columns of up to 128, 224, 352 and 544 points have a register-resident form (LM points per
+// lane and segment, NC groups of 32 points), longer ones (LM = 0) keep their segments in
+// shared memory.
+static int fin_lm(int nR) {
+  return nR <= 128 ? 5 : nR <= 224 ? 7 : nR <= 352 ? 11 : nR <= 544 ? 17 : 0;
+}
+
+constexpr size_t kFinRoom = 200 * 1024;  // dynamic shared memory a CTA of these kernels may take
+
+static const void* finalize_fn(int lm) {
+  return lm == 5    ? (const void*)finalize_kernel<5, 4>
+         : lm == 7  ? (const void*)finalize_kernel<7, 7>
+         : lm == 11 ? (const void*)finalize_kernel<11, 11>
+         : lm == 17 ? (const void*)finalize_kernel<17, 17>
+                    : (const void*)finalize_kernel<0, 1>;
+}
+
+// Launch shape for P columns of nR points from n_part partial sums, once per plan: eight
+// warps per CTA, fewer only where the shared rows of a long column need it.
+static int finalize_shape(int64_t P, int nR, int n_part, int n_sm, FinLaunch* L) {
+  const int lm = fin_lm(nR);
+  const auto bytes = [&](int w) { return fin_smem<1>(nR, w * (1 + (lm ? 0 : 1) + n_part)); };
+  int warps = 8;
+  while (warps > 1 && bytes(warps) > kFinRoom) warps /= 2;
+  MQCT_ARG_CHECK(bytes(warps) <= kFinRoom, "nR=%d with %d partial sums beyond the finalize", nR,
+                 n_part);
+  L->fn = finalize_fn(lm);
+  L->warps = warps;
+  L->smem = bytes(warps);
+  MQCT_CUDA_TRY(cudaFuncSetAttribute(L->fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)kFinRoom));
+  int per_sm = 1;
+  MQCT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, L->fn, 32 * warps, L->smem));
+  L->grid = (unsigned)std::min<int64_t>(P, (int64_t)n_sm * std::max(per_sm, 1));
+  return MQCT_OK;
+}
+
+static int launch_finalize(const FinLaunch& L, int64_t P, FinGrid g, const int* k_to_row,
+                           const double* part, int n_part, int64_t part_stride, int ldp,
+                           double scale, cudaStream_t st) {
+  void* args[] = {&P, &g, &k_to_row, &part, &n_part, &part_stride, &ldp, &scale};
+  MQCT_CUDA_TRY(cudaLaunchKernel(L.fn, dim3(L.grid), dim3(32 * L.warps), args, L.smem, st));
+  return MQCT_OK;
 }
 
 // (b) spline_kernel: clamped cubic spline with finite-difference end slopes
@@ -618,7 +575,7 @@ static double clebsch_gordan(int j1, int m1, int j2, int m2, int J, int M) {
   return sum;
 }
 
-// Grid-only coefficients of finalize_kernel's spline fit (5 x nR, see there).
+// Grid-only coefficients of the spline fit of finalize.cuh (5 x nR, see FinGrid).
 static std::vector<double> spline_grid_coefs(const std::vector<double>& Rh) {
   const int nR = (int)Rh.size();
   std::vector<double> gc(5 * (size_t)nR, 0.0);
@@ -740,6 +697,11 @@ int MatrixPlan::init(const mqct_sys_t* sys, const int32_t* ind_mat, int64_t P_, 
   cut = mij_cut * kCmToHartree;
   MQCT_CUDA_TRY(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
   for (auto& e : ev) MQCT_CUDA_TRY(cudaEventCreate(&e));
+  {
+    int dev = 0;
+    MQCT_CUDA_TRY(cudaGetDevice(&dev));
+    MQCT_CUDA_TRY(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
+  }
 
   // --- states -> m-blocks
   std::map<int, std::vector<int>> by_m;
@@ -973,6 +935,8 @@ int MatrixPlan::init(const mqct_sys_t* sys, const int32_t* ind_mat, int64_t P_, 
     int rc2 = tc_init();
     if (rc2) return rc2;
   }
+  rc = finalize_shape(P, nR, precision == MQCT_PREC_FP64 ? 1 : tc_splits, n_sm, &fin);
+  if (rc) return rc;
   MQCT_CUDA_TRY(cudaStreamSynchronize(stream));
   return MQCT_OK;
 }
@@ -1064,26 +1028,22 @@ int MatrixPlan::execute(double* d_mat, double* d_y2, int32_t* d_skipped) {
   int rc = run_basis_and_pes();
   if (rc) return rc;
   MQCT_CUDA_TRY(cudaEventRecord(ev[1], stream));
-  const size_t fin_smem = sizeof(double) * 2 * (size_t)nR;
+  const FinGrid fg{nR, ir1, ir2, cut, d_spl_fin.p, d_mat, d_skipped, d_y2};
   if (precision == MQCT_PREC_FP64) {
     dim3 g((n_rows + F_TM - 1) / F_TM, (nR + F_TN - 1) / F_TN);
     contract_fp64_kernel<<<g, 256, 0, stream>>>(n_rows, G2, nR, d_rowa.p, d_rowb.p, d_psi.p,
                                                 d_W.p, ldw, n_alpha, d_walpha.p, d_acc.p);
     MQCT_CUDA_TRY(cudaGetLastError());
     MQCT_CUDA_TRY(cudaEventRecord(ev[2], stream));
-    finalize_kernel<double><<<(unsigned)P, 128, fin_smem, stream>>>(
-        P, nR, d_k2r.p, d_acc.p, 1, 0, nR, kCmToHartree, nullptr, ir1, ir2, cut, d_spl_fin.p,
-        d_mat, d_skipped, d_y2);
-    MQCT_CUDA_TRY(cudaGetLastError());
+    rc = launch_finalize(fin, P, fg, d_k2r.p, d_acc.p, 1, 0, nR, kCmToHartree, stream);
   } else {
     rc = tc_execute();
     if (rc) return rc;
     MQCT_CUDA_TRY(cudaEventRecord(ev[2], stream));
-    finalize_kernel<double><<<(unsigned)P, 128, fin_smem, stream>>>(
-        P, nR, d_k2r.p, d_part.p, tc_splits, (int64_t)n_rows * tc_ldp, tc_ldp, kCmToHartree,
-        nullptr, ir1, ir2, cut, d_spl_fin.p, d_mat, d_skipped, d_y2);
-    MQCT_CUDA_TRY(cudaGetLastError());
+    rc = launch_finalize(fin, P, fg, d_k2r.p, d_part.p, tc_splits, (int64_t)n_rows * tc_ldp, tc_ldp,
+                         kCmToHartree, stream);
   }
+  if (rc) return rc;
   MQCT_CUDA_TRY(cudaEventRecord(ev[3], stream));
   return MQCT_OK;
 }
@@ -1600,12 +1560,13 @@ __device__ inline double rotor_sum(int jpp, int l, int jp, int nju, const double
 // only: they are formed once per (channel pair, term) and per (pair, distinct
 // (l1, l2, l)), and A in the contraction, with the products in the order above.
 
-// K[(c' n_ch + c'') n_terms + t].
+// FK[(c' n_ch + c'') n_terms + t] = fac_t K.
 __global__ void expansion_k_kernel(int n_ch, int n_terms, const int* __restrict__ ch_j1,
                                    const int* __restrict__ ch_j2,
                                    const double* __restrict__ vec1, int ldv1,
                                    const double* __restrict__ vec2, int ldv2,
-                                   const int* __restrict__ lab5, double* __restrict__ K) {
+                                   const int* __restrict__ lab5,
+                                   const double* __restrict__ fac, double* __restrict__ FK) {
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (int64_t)n_ch * n_ch * n_terms) return;
   const int t = (int)(idx % n_terms);
@@ -1628,7 +1589,7 @@ __global__ void expansion_k_kernel(int n_ch, int n_terms, const int* __restrict_
       if (s1 != 0.0) kt += phase * s1 * rotor_sum(j2pp, l2, j2p, n2, v2p, v2pp);
     }
   }
-  K[idx] = kt;
+  FK[idx] = fac[t] * kt;
 }
 
 // M3[k n_u + u] for the distinct (l1, l2, l) = lll[3u .. 3u+2].
@@ -1759,7 +1720,6 @@ __global__ void expansion_identical_kernel(int64_t P, int n_terms, const int* __
   A[idx] = a;
 }
 
-// M[k * nR + i] = sum_t A[k * n_terms + t] T[t * nR + i] from stored coefficients.
 // Coefficients of a rotor and an atom (EXPANSION_MATRIX_ELEMENT, SYS_TYPE 1 and 4,
 // MQCT_SOURCE_CODES/pot_comp.f:6551-6622 and 6955-7075), one thread per (pair, term):
 //   A = sqrt((2j'+1)/(2j''+1)) sqrt((2l+1)/4pi) <j' m l 0|j'' m> S,
@@ -1806,20 +1766,6 @@ __global__ void expansion_atom_kernel(int64_t P, int n_terms, const int* __restr
         cg_dev(jp, m, l, 0, jpp, m) * S;
   }
   A[idx] = a;
-}
-
-__global__ void __launch_bounds__(128)
-expansion_contract_a_kernel(int n_terms, int nR, const double* __restrict__ A,
-                            const double* __restrict__ T, double* __restrict__ M) {
-  extern __shared__ double ex_a[];
-  const int64_t k = blockIdx.x;
-  for (int t = threadIdx.x; t < n_terms; t += blockDim.x) ex_a[t] = A[k * n_terms + t];
-  __syncthreads();
-  for (int i = threadIdx.x; i < nR; i += blockDim.x) {
-    double s = 0.0;
-    for (int t = 0; t < n_terms; ++t) s = fma(ex_a[t], T[(size_t)t * nR + i], s);
-    M[k * nR + i] = s;
-  }
 }
 
 // Clebsch-Gordan tables for expansion_m3_table_kernel, filled by cg_dev (the same
@@ -1910,32 +1856,314 @@ __global__ void expansion_m3_table_kernel(int64_t P, int n_u, const int* __restr
   M3[idx] = m3;
 }
 
-// M[k * nR + i] = sum_t A[k, t] T[t * nR + i] (fixed order); one CTA per pair: the
-// pair's coefficients A[k, t] = fac_t K M3 c_k into shared memory, then threads along R
-// (coalesced T rows).  fac_t = pref sqrt((2l1+1)(2l2+1)), u_t the term's (l1, l2, l).
-__global__ void __launch_bounds__(128)
-expansion_contract_kernel(int n_ch, int n_terms, int n_u, int nR, const int* __restrict__ ind_mat,
-                          const int* __restrict__ st_chan, const int* __restrict__ ch_j1,
-                          const int* __restrict__ ch_j2, const double* __restrict__ K,
-                          const double* __restrict__ M3, const double* __restrict__ fac,
-                          const int* __restrict__ term_u, const double* __restrict__ T,
-                          double* __restrict__ M) {
-  extern __shared__ double ex_a[];
-  const int64_t k = blockIdx.x;
-  const int cp = st_chan[ind_mat[2 * k] - 1], cpp = st_chan[ind_mat[2 * k + 1] - 1];
-  const int j1p = ch_j1[cp], j2p = ch_j2[cp], j1pp = ch_j1[cpp], j2pp = ch_j2[cpp];
-  const double c1 = sqrt((2.0 * j1pp + 1.0) / (2.0 * j1p + 1.0));
-  const double c2 = sqrt((2.0 * j2pp + 1.0) / (2.0 * j2p + 1.0));
-  const double* Kc = K + ((int64_t)cp * n_ch + cpp) * n_terms;
-  const double* Mk = M3 + k * n_u;
-  for (int t = threadIdx.x; t < n_terms; t += blockDim.x)
-    ex_a[t] = fac[t] * Kc[t] * Mk[term_u[t]] * c1 * c2;
+// Coefficients of the expansion: stored whole (A, n_terms per pair: identical partners,
+// rotor + atom), or A[k, t] = FK M3 c1 c2 with FK = fac_t K of the pair's channels, fac_t =
+// pref sqrt((2l1+1)(2l2+1)), and term_u[t] the term's distinct (l1, l2, l).
+struct ExpCoef {
+  int n_terms, n_u;
+  const double* A;
+  const double* FK;
+  const double* M3;
+  const int* term_u;
+};
+// A group of pairs of one channel pair: its row of FK and rotor factors.
+struct ExGroup {
+  int64_t k_off;
+  double c1, c2;
+};
+// Terms whose coefficients a warp lists at a time: 128 (their loads in flight together) where
+// the lists of the CTA's warps leave the L1 cache its room for T.
+__host__ __device__ constexpr int ex_blk(int G) { return G >= 4 ? 32 : 128; }
+// Columns a warp finishes together (see fin_columns): as its registers allow.
+__host__ __device__ constexpr int ex_cols(int LM, int G) {
+  return LM == 5 ? (G < 4 ? G : 4) : LM == 7 ? 2 : 1;
+}
+constexpr size_t kExpRoom = 226 * 1024;  // dynamic shared memory of a CTA, T included
+// Pairs a warp sums together: as many as its registers hold sums for (the reads of T and the
+// list are shared by them), two where there are too few pairs to give every warp more.
+static int ex_group(int nR, int64_t P, int n_sm) {
+  const int lm = fin_lm(nR);
+  const int g = lm == 5 ? 8 : lm == 7 ? 4 : lm == 11 ? 2 : 1;
+  return P >= (int64_t)n_sm * 16 * 2 * g ? g : std::min(g, 2);
+}
+
+// Pairs in the order of their two channels, each channel pair's pairs from a multiple of G
+// places on (-1: an empty place), so that the G pairs of a warp have the same zeros among
+// their coefficients.  count: one entry per channel pair, zeroed before; after the scan the
+// place where each channel pair begins, moved on by the scatter (the order inside a channel
+// pair is that of arrival; no result depends on it).
+__global__ void ex_count_kernel(int64_t P, const int* __restrict__ ind_mat,
+                                const int* __restrict__ st_chan, int n_ch, int* __restrict__ count) {
+  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= P) return;
+  atomicAdd(count + (int64_t)st_chan[ind_mat[2 * k] - 1] * n_ch + st_chan[ind_mat[2 * k + 1] - 1], 1);
+}
+// Exclusive scan of the counts rounded up to G, one CTA of 1024 threads; total[0] the sum.
+__global__ void __launch_bounds__(1024) ex_scan_kernel(int64_t n, int G, int* __restrict__ count,
+                                                       int* __restrict__ total) {
+  __shared__ int part[32];
+  __shared__ int carry_s;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (threadIdx.x == 0) carry_s = 0;
   __syncthreads();
-  for (int i = threadIdx.x; i < nR; i += blockDim.x) {
-    double s = 0.0;
-    for (int t = 0; t < n_terms; ++t) s = fma(ex_a[t], T[(size_t)t * nR + i], s);
-    M[k * nR + i] = s;
+  for (int64_t i0 = 0; i0 < n; i0 += 1024) {
+    const int64_t i = i0 + threadIdx.x;
+    const int v = i < n ? (count[i] + G - 1) / G * G : 0;
+    int x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int p = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += p;
+    }
+    if (lane == 31) part[w] = x;
+    __syncthreads();
+    if (w == 0) {
+      int q = part[lane];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int p = __shfl_up_sync(0xffffffffu, q, o);
+        if (lane >= o) q += p;
+      }
+      part[lane] = q;
+    }
+    __syncthreads();
+    const int before = carry_s + (w ? part[w - 1] : 0) + x - v;
+    if (i < n) count[i] = before;
+    __syncthreads();
+    if (threadIdx.x == 0) carry_s += part[31];
+    __syncthreads();
   }
+  if (threadIdx.x == 0) total[0] = carry_s;
+}
+__global__ void ex_scatter_kernel(int64_t P, const int* __restrict__ ind_mat,
+                                  const int* __restrict__ st_chan, int n_ch, int* __restrict__ count,
+                                  int* __restrict__ order) {
+  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= P) return;
+  const int64_t c = (int64_t)st_chan[ind_mat[2 * k] - 1] * n_ch + st_chan[ind_mat[2 * k + 1] - 1];
+  order[atomicAdd(count + c, 1)] = (int)k;
+}
+
+// The groups' rows of FK and rotor factors.
+__global__ void ex_group_kernel(int n_groups, int G, const int* __restrict__ order,
+                                const int* __restrict__ ind_mat, const int* __restrict__ st_chan,
+                                const int* __restrict__ ch_j1, const int* __restrict__ ch_j2,
+                                int n_ch, int n_terms, ExGroup* __restrict__ grp) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n_groups) return;
+  const int64_t k = order[(int64_t)i * G];  // the first place of a group is never empty
+  const int cp = st_chan[ind_mat[2 * k] - 1], cpp = st_chan[ind_mat[2 * k + 1] - 1];
+  grp[i].k_off = ((int64_t)cp * n_ch + cpp) * n_terms;
+  grp[i].c1 = sqrt((2.0 * ch_j1[cpp] + 1.0) / (2.0 * ch_j1[cp] + 1.0));
+  grp[i].c2 = sqrt((2.0 * ch_j2[cpp] + 1.0) / (2.0 * ch_j2[cp] + 1.0));
+}
+
+// Mat_el, flags and y2 of each pair from M(R) = e_unit sum_t A[k, t] T[t, R], one warp per G
+// pairs of one channel pair on a persistent grid.  The triangle rules and the rotor symmetry
+// make about half of a pair's coefficients exactly zero (asymmetric top + homonuclear
+// diatom), the same ones for the pairs of a channel pair: the warp forms 32 terms'
+// coefficients at a time, lists the terms where one of its pairs has a nonzero one (in term
+// order) and adds only their rows of T, the lanes along R with the sums in registers.  What
+// bounds it is instruction issue and FP64, so a row read, its address and its bounds checks
+// serve G pairs, and Q columns are finished together.  T (100 KB at 128 terms x 101 points)
+// is kept in shared memory: left to L1, which the other reads and the output pass through,
+// half of its reads missed.  The order of the sums is that of the full sum, and the skipped
+// products are exact zeros, so the result is the same bit for bit; a T with an infinity or NaN
+// (0 x inf is NaN) takes the full sum, decided once per CTA from a look at all of T.  The
+// columns then go straight to the cut-off and the spline (finalize.cuh) instead of through
+// global memory.
+template <int LM, int NC, int G, bool TS>
+__global__ void __launch_bounds__(G >= 4 ? 384 : 512, 1)
+expansion_kernel(int n_groups, FinGrid g, ExpCoef ex, const int* __restrict__ order,
+                 const ExGroup* __restrict__ grp, const double* __restrict__ T, double e_unit,
+                 int* __restrict__ queue) {
+  constexpr int BLK = ex_blk(G), Q = ex_cols(LM, G);
+  extern __shared__ double fin_sm[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int nR = g.nR, ld = fin_len(nR), n_terms = ex.n_terms;
+  constexpr int ROWS = LM ? G : 2;   // shared rows of a warp: its columns, or column and scratch
+  double* cols = fin_sm + kFinMul + (size_t)ld * (4 + warp * ROWS);
+  double* lists = fin_sm + kFinMul + (size_t)ld * (4 + nw * ROWS);
+  double* la = lists + (size_t)warp * BLK * G;
+  int* lt = reinterpret_cast<int*>(lists + (size_t)nw * BLK * G) + warp * BLK;
+  double* Ts = lists + (size_t)nw * BLK * G + (size_t)nw * BLK / 2;
+  // The warps take groups from a queue (the channel pairs differ several-fold in cost), the
+  // first round without it; a group's pairs and factors are loaded one group ahead.
+  const int n_warps = gridDim.x * nw;
+  int gi = warp * gridDim.x + blockIdx.x;
+  int n_k[G];
+  ExGroup n_g{0, 1.0, 1.0};
+  auto look = [&](int i) {
+    if (i >= n_groups) return;
+#pragma unroll
+    for (int q = 0; q < G; ++q) n_k[q] = order[i * G + q];
+    if (!ex.A) n_g = grp[i];
+  };
+  look(gi);
+  bool odd = false;
+#pragma unroll 8
+  for (int q = threadIdx.x; q < n_terms * nR; q += blockDim.x) {
+    const double t = __ldg(T + q);
+    if (TS) Ts[q] = t;
+    odd |= !isfinite(t);
+  }
+  // lanes beyond the last point read on into the next row, those of the last row into zeros
+  if (TS)
+    for (int q = threadIdx.x; q < 32 * NC; q += blockDim.x) Ts[n_terms * nR + q] = 0.0;
+  FinLane<LM> f;
+  fin_init<LM>(g, fin_sm, f);
+  const double* coef = fin_sm + kFinMul;
+  const bool full = __syncthreads_or(odd) != 0;
+  while (gi < n_groups) {
+    const double c1 = n_g.c1, c2 = n_g.c2;
+    const double* FK = ex.FK + n_g.k_off;
+    int k[G];
+#pragma unroll
+    for (int q = 0; q < G; ++q) k[q] = n_k[q];
+    int nx = n_groups;
+    if (n_groups > n_warps) {
+      if (lane == 0) nx = n_warps + atomicAdd(queue, 1);
+      nx = __shfl_sync(0xffffffffu, nx, 0);
+    }
+    gi = nx;
+    __syncwarp();                      // the previous columns are done with cols
+    for (int i0 = 0; i0 < nR; i0 += 32 * NC) {
+      double s[G][NC];
+#pragma unroll
+      for (int q = 0; q < G; ++q)
+#pragma unroll
+        for (int c = 0; c < NC; ++c) s[q][c] = 0.0;
+      for (int t0 = 0; t0 < n_terms; t0 += BLK) {
+        int cnt = 0;
+#pragma unroll
+        for (int j = 0; j < BLK / 32; ++j) {
+          const int t = t0 + 32 * j + lane;
+          double a[G];
+          bool use = full && t < n_terms;
+          if (t < n_terms) {
+            if (ex.A) {
+#pragma unroll
+              for (int q = 0; q < G; ++q) {
+                a[q] = k[q] >= 0 ? ex.A[(int64_t)k[q] * n_terms + t] : 0.0;
+                use |= !(a[q] == 0.0);
+              }
+            } else {
+              const double fk = FK[t];
+              const int u = ex.term_u[t];
+#pragma unroll
+              for (int q = 0; q < G; ++q) {
+                a[q] = k[q] >= 0 ? fk * ex.M3[(int64_t)k[q] * ex.n_u + u] * c1 * c2 : 0.0;
+                use |= !(a[q] == 0.0);
+              }
+            }
+          }
+          const unsigned b = __ballot_sync(0xffffffffu, use);
+          if (use) {
+            const int at = cnt + __popc(b & ((1u << lane) - 1u));
+#pragma unroll
+            for (int q = 0; q < G; ++q) la[at * G + q] = a[q];
+            lt[at] = t * nR;
+          }
+          cnt += __popc(b);
+        }
+        __syncwarp();
+#pragma unroll 2
+        for (int e = 0; e < cnt; ++e) {
+          double a[G], tv[NC];
+          if constexpr (G % 2 == 0) {
+#pragma unroll
+            for (int q = 0; q < G; q += 2) {
+              const double2 v = *reinterpret_cast<const double2*>(la + e * G + q);
+              a[q] = v.x;
+              a[q + 1] = v.y;
+            }
+          } else {
+            a[0] = la[e];
+          }
+          const int o = lt[e] + i0 + lane;
+#pragma unroll
+          for (int c = 0; c < NC; ++c)
+            tv[c] = TS ? Ts[o + 32 * c] : i0 + lane + 32 * c < nR ? __ldg(T + o + 32 * c) : 0.0;
+#pragma unroll
+          for (int q = 0; q < G; ++q)
+#pragma unroll
+            for (int c = 0; c < NC; ++c) s[q][c] = fma(a[q], tv[c], s[q][c]);
+        }
+        __syncwarp();
+      }
+      if (i0 == 0) look(gi);
+      if constexpr (LM == 0) {  // G = 1: the column is finished after its last group of points
+#pragma unroll
+        for (int c = 0; c < NC; ++c)
+          if (i0 + lane + 32 * c < nR) cols[i0 + lane + 32 * c] = s[0][c] * e_unit;
+      } else {
+#pragma unroll
+        for (int q = 0; q < G; ++q)
+#pragma unroll
+          for (int c = 0; c < NC; ++c)
+            if (lane + 32 * c < nR) cols[q * ld + lane + 32 * c] = s[q][c] * e_unit;
+      }
+    }
+    __syncwarp();
+    if constexpr (LM > 0) {
+#pragma unroll 1
+      for (int q0 = 0; q0 < G; q0 += Q) {
+        int64_t kq[Q];
+#pragma unroll
+        for (int r = 0; r < Q; ++r) {
+          int v = k[r];
+#pragma unroll
+          for (int o = Q; o < G; o += Q) v = q0 == o ? k[o + r] : v;
+          kq[r] = v;
+        }
+        if (kq[0] < 0) break;            // empty places come last
+        fin_columns<LM, NC, Q>(g, f, coef, cols + q0 * ld, cols, kq);
+      }
+    }
+    if constexpr (LM == 0) {
+      const int64_t kq[1] = {k[0]};
+      __syncwarp();
+      fin_columns<LM, 1, 1>(g, f, coef, cols, cols + ld, kq);
+    }
+  }
+  // the last warp leaves the queue as it found it
+  if (n_groups > n_warps && lane == 0) {
+    __threadfence();
+    if (atomicAdd(queue + 1, 1) == n_warps - 1) {
+      queue[0] = 0;
+      queue[1] = 0;
+    }
+  }
+}
+
+// One CTA per SM: T is read once per SM, into shared memory where it fits.
+template <bool TS>
+static const void* expansion_fn(int lm, int G) {
+  return lm == 5    ? (G == 8 ? (const void*)expansion_kernel<5, 4, 8, TS>
+                               : (const void*)expansion_kernel<5, 4, 2, TS>)
+         : lm == 7  ? (G == 4 ? (const void*)expansion_kernel<7, 7, 4, TS>
+                              : (const void*)expansion_kernel<7, 7, 2, TS>)
+         : lm == 11 ? (const void*)expansion_kernel<11, 11, 2, TS>
+         : lm == 17 ? (const void*)expansion_kernel<17, 17, 1, TS>
+                    : (const void*)expansion_kernel<0, 16, 1, TS>;
+}
+static int expansion_shape(int n_groups, int nR, int n_terms, int G, int n_sm, FinLaunch* L) {
+  const int lm = fin_lm(nR), rows = lm ? G : 2;
+  const auto bytes = [&](int w) {
+    return fin_smem<1>(nR, w * rows) + (size_t)w * ex_blk(G) * (8 * G + 4);
+  };
+  int warps = G >= 4 ? 12 : 16;
+  while (warps > 1 && bytes(warps) > kFinRoom) warps /= 2;
+  L->warps = warps;
+  L->smem = bytes(warps);
+  const size_t with_t = L->smem + sizeof(double) * ((size_t)n_terms * nR + 32 * 17);
+  const bool ts = with_t <= kExpRoom;
+  if (ts) L->smem = with_t;
+  L->fn = ts ? expansion_fn<true>(lm, G) : expansion_fn<false>(lm, G);
+  L->grid = (unsigned)std::max(1, std::min(n_groups, n_sm));
+  MQCT_CUDA_TRY(cudaFuncSetAttribute(L->fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)kExpRoom));
+  return MQCT_OK;
 }
 
 namespace {
@@ -1957,8 +2185,50 @@ struct ExpansionPlan {
   bool a_stored = false;  // coefficients stored whole in d_A (identical partners, types 1 and 4)
   std::vector<double> sym_top_vec;  // SYS_TYPE 9: the second rotor's vectors
   mqct_sys_t sys_map{};
-  DevBuf<int> d_k2r, d_ind, d_chan, d_j1, d_j2, d_term_u;
-  DevBuf<double> d_K, d_M3, d_fac, d_M, d_gc, d_A;
+  DevBuf<int> d_ind, d_chan, d_j1, d_j2, d_term_u;
+  DevBuf<double> d_K, d_M3, d_fac, d_gc, d_A;
+  DevBuf<int> d_order;        // pairs grouped by channel pair (expansion_kernel)
+  DevBuf<ExGroup> d_grp;
+  DevBuf<int> d_queue;        // next group, warps done (zero between launches)
+  int n_groups = 0;
+  FinLaunch fin;
+
+  // Groups the pairs (d_ind, d_chan already queued on st) and shapes the launch.
+  int group_pairs() {
+    int dev = 0, n_sm = 0;
+    MQCT_CUDA_TRY(cudaGetDevice(&dev));
+    MQCT_CUDA_TRY(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
+    const int G = ex_group(nR, P, n_sm);
+    const int64_t nc2 = (int64_t)n_ch * n_ch;
+    MQCT_ARG_CHECK(nc2 < ((int64_t)1 << 31) - 1, "%d channels beyond the expansion build", n_ch);
+    // places: the pairs, and at most G - 1 empty ones per channel pair that has pairs
+    const int64_t cap = P + (G - 1) * std::min<int64_t>(P, nc2);
+    MQCT_ARG_CHECK(cap < ((int64_t)1 << 31), "too many pairs");
+    DevBuf<int> cnt;
+    MQCT_CUDA_TRY(cnt.alloc((size_t)nc2 + 1));
+    MQCT_CUDA_TRY(d_order.alloc((size_t)cap));
+    MQCT_CUDA_TRY(cudaMemsetAsync(cnt.p, 0, sizeof(int) * (size_t)(nc2 + 1), st));
+    MQCT_CUDA_TRY(cudaMemsetAsync(d_order.p, 0xff, sizeof(int) * (size_t)cap, st));
+    const unsigned gb = (unsigned)((P + 255) / 256);
+    ex_count_kernel<<<gb, 256, 0, st>>>(P, d_ind.p, d_chan.p, n_ch, cnt.p);
+    ex_scan_kernel<<<1, 1024, 0, st>>>(nc2, G, cnt.p, cnt.p + nc2);
+    int total = 0;
+    MQCT_CUDA_TRY(cudaMemcpyAsync(&total, cnt.p + nc2, sizeof(int), cudaMemcpyDeviceToHost, st));
+    ex_scatter_kernel<<<gb, 256, 0, st>>>(P, d_ind.p, d_chan.p, n_ch, cnt.p, d_order.p);
+    MQCT_CUDA_TRY(cudaGetLastError());
+    MQCT_CUDA_TRY(cudaStreamSynchronize(st));  // total; the counts are released on return
+    n_groups = total / G;
+    if (!a_stored) {
+      MQCT_CUDA_TRY(d_grp.alloc((size_t)n_groups));
+      ex_group_kernel<<<(unsigned)((n_groups + 255) / 256), 256, 0, st>>>(
+          n_groups, G, d_order.p, d_ind.p, d_chan.p, d_j1.p, d_j2.p, n_ch, n_terms, d_grp.p);
+      MQCT_CUDA_TRY(cudaGetLastError());
+      MQCT_CUDA_TRY(cudaStreamSynchronize(st));
+    }
+    MQCT_CUDA_TRY(d_queue.alloc(2));
+    MQCT_CUDA_TRY(cudaMemsetAsync(d_queue.p, 0, 2 * sizeof(int), st));
+    return expansion_shape(n_groups, nR, n_terms, G, n_sm, &fin);
+  }
 
   ~ExpansionPlan() {
     for (auto& e : ev)
@@ -1983,10 +2253,6 @@ struct ExpansionPlan {
     MQCT_CUDA_TRY(d_ind.upload(ind_mat, 2 * (size_t)P, st));
     std::vector<double> Rh(R, R + nR);
     MQCT_CUDA_TRY(d_gc.upload(spline_grid_coefs(Rh), st));
-    std::vector<int> k2r(P);
-    for (int64_t k = 0; k < P; ++k) k2r[k] = (int)k;
-    MQCT_CUDA_TRY(d_k2r.upload(k2r, st));
-    MQCT_CUDA_TRY(d_M.alloc((size_t)P * nR));
     ir1 = nearest_index(Rh, r_cut1);
     ir2 = nearest_index(Rh, r_cut2);
     cut_hartree = mij_cutoff_cm * kCmToHartree;
@@ -2082,8 +2348,7 @@ struct ExpansionPlan {
         d_A.p);
     MQCT_CUDA_TRY(cudaGetLastError());
     MQCT_CUDA_TRY(cudaEventRecord(ev[1], st));
-    MQCT_CUDA_TRY(cudaStreamSynchronize(st));
-    return MQCT_OK;
+    return group_pairs();  // waits for st: the set-up buffers are released on return
   }
 
   int init(const mqct_sys_t* sys, const int32_t* ind_mat, int64_t P_, const double* R,
@@ -2277,10 +2542,6 @@ struct ExpansionPlan {
     MQCT_CUDA_TRY(d_fac.upload(fac, st));
     std::vector<double> Rh(R, R + nR);
     MQCT_CUDA_TRY(d_gc.upload(spline_grid_coefs(Rh), st));
-    std::vector<int> k2r(P);
-    for (int64_t k = 0; k < P; ++k) k2r[k] = (int)k;
-    MQCT_CUDA_TRY(d_k2r.upload(k2r, st));
-    MQCT_CUDA_TRY(d_M.alloc((size_t)P * nR));
     if (!ident) {
       MQCT_CUDA_TRY(d_K.alloc((size_t)n_ch * n_ch * n_terms));
       MQCT_CUDA_TRY(d_M3.alloc((size_t)P * n_u));
@@ -2320,8 +2581,7 @@ struct ExpansionPlan {
           d_vec1.p, d_vec2.p, ldv1, d_lab.p, d_A.p);
       MQCT_CUDA_TRY(cudaGetLastError());
       MQCT_CUDA_TRY(cudaEventRecord(ev[1], st));
-      MQCT_CUDA_TRY(cudaStreamSynchronize(st));
-      return MQCT_OK;
+      return group_pairs();  // waits for st: the set-up buffers are released on return
     }
     const int64_t n_k = (int64_t)n_ch * n_ch * n_terms, n_m3 = P * n_u;
     // table sizes from the actual j and l ranges
@@ -2338,7 +2598,7 @@ struct ExpansionPlan {
     DevBuf<double> d_tab;  // the four tables in one allocation
     MQCT_CUDA_TRY(cudaEventRecord(ev[0], st));
     expansion_k_kernel<<<(unsigned)((n_k + 127) / 128), 128, 0, st>>>(
-        n_ch, n_terms, d_j1.p, d_j2.p, d_vec1.p, ldv1, d_vec2.p, ldv2, d_lab.p, d_K.p);
+        n_ch, n_terms, d_j1.p, d_j2.p, d_vec1.p, ldv1, d_vec2.p, ldv2, d_lab.p, d_fac.p, d_K.p);
     MQCT_CUDA_TRY(cudaGetLastError());
     if (tables) {
       const int64_t n_st = (int64_t)n_states * (2 * J1 + 1), n_lt = (int64_t)n_u * (2 * Lm + 1);
@@ -2362,8 +2622,7 @@ struct ExpansionPlan {
     }
     MQCT_CUDA_TRY(cudaGetLastError());
     MQCT_CUDA_TRY(cudaEventRecord(ev[1], st));
-    MQCT_CUDA_TRY(cudaStreamSynchronize(st));  // the set-up buffers are released on return
-    return MQCT_OK;
+    return group_pairs();  // waits for st: the set-up buffers are released on return
   }
 
   // Mat_el (Hartree), y2 and the MIJ_CUTOFF flags from radial terms d_terms
@@ -2372,18 +2631,13 @@ struct ExpansionPlan {
     MQCT_ARG_CHECK(d_terms && d_mat && d_sk, "null argument");
     MQCT_ARG_CHECK(e_unit > 0.0, "e_unit must be positive");
     MQCT_CUDA_TRY(cudaEventRecord(ev[2], st));
-    if (a_stored)
-      expansion_contract_a_kernel<<<(unsigned)P, 128, sizeof(double) * (size_t)n_terms, st>>>(
-          n_terms, nR, d_A.p, d_terms, d_M.p);
-    else
-      expansion_contract_kernel<<<(unsigned)P, 128, sizeof(double) * (size_t)n_terms, st>>>(
-          n_ch, n_terms, n_u, nR, d_ind.p, d_chan.p, d_j1.p, d_j2.p, d_K.p, d_M3.p, d_fac.p,
-          d_term_u.p, d_terms, d_M.p);
-    MQCT_CUDA_TRY(cudaGetLastError());
-    finalize_kernel<double><<<(unsigned)P, 128, sizeof(double) * 2 * (size_t)nR, st>>>(
-        P, nR, d_k2r.p, d_M.p, 1, 0, nR, e_unit, nullptr, ir1, ir2, cut_hartree, d_gc.p, d_mat,
-        d_sk, d_y2);
-    MQCT_CUDA_TRY(cudaGetLastError());
+    FinGrid fg{nR, ir1, ir2, cut_hartree, d_gc.p, d_mat, d_sk, d_y2};
+    ExpCoef ex{n_terms, n_u, a_stored ? d_A.p : nullptr, d_K.p, d_M3.p, d_term_u.p};
+    const int* order = d_order.p;
+    const ExGroup* grp = d_grp.p;
+    int* queue = d_queue.p;
+    void* args[] = {&n_groups, &fg, &ex, &order, &grp, &d_terms, &e_unit, &queue};
+    MQCT_CUDA_TRY(cudaLaunchKernel(fin.fn, dim3(fin.grid), dim3(32 * fin.warps), args, fin.smem, st));
     MQCT_CUDA_TRY(cudaEventRecord(ev[3], st));
     return MQCT_OK;
   }

@@ -12,6 +12,14 @@ namespace mqct {
 int surrogate_predict_on(void* sur, const float* X, int64_t n, double* v_out, cudaStream_t st);
 void surrogate_feature_map(const void* sur, int* sys_type, double* r_c, double* r_s);
 
+// Launch shape of the finalize and expansion kernels for one plan.
+struct FinLaunch {
+  const void* fn = nullptr;
+  int warps = 8;
+  unsigned grid = 1;
+  size_t smem = 0;
+};
+
 // Per-plan state of the tcgen05 path (contract_tc.cu).
 struct TcInfo {
   int n_chunks = 0, chunks_per_split = 1, npad = 0, nbmax = 0;
@@ -41,6 +49,8 @@ struct MatrixPlan {
   int n_alpha = 0;   // explicit alpha grid points (0: analytic 2*pi)
   int ldv = 1;
   int ir1 = 0, ir2 = 0;
+  int n_sm = 148;
+  FinLaunch fin;
   double cut = 0.0;
   int pes_kind = 0, pes_n_terms = 0, pes_n_sites1 = 0, pes_n_sites2 = 0;
   std::vector<double> Rh, h_beta, h_gamma, h_wt, h_alpha, h_walpha;
