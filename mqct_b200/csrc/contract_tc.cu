@@ -202,32 +202,34 @@ __device__ __forceinline__ void split8(const float (&x)[8], uint4& h, uint4& l) 
   }
 }
 
-// F16x3 column scaling: one CTA per radial column i finds max_g |W[g, i]| and
-// writes the exponent s_i with max * 2^s_i in [2^13, 2^14) and the factor
-// 2^-(s_i + kXScaleExp) that undoes both scalings.
+// F16x3 column scaling: max_g |W[g, i]| of every radial column (its bits; non-negative doubles
+// order as integers), lanes along R over a slice of the grid.  The exponent s_i brings it to
+// [2^13, 2^14); 2^-(s_i + kXScaleExp) undoes both scalings (tc_bimage_kernel).
 constexpr int kXScaleExp = 14;
-__global__ void tc_wscale_kernel(const double* __restrict__ W, int ldw, int G2,
-                                 int* __restrict__ wexp, double* __restrict__ col_scale) {
-  __shared__ double red[32];
-  const int i = blockIdx.x;
+__global__ void __launch_bounds__(256)
+tc_wmax_kernel(const double* __restrict__ W, int ldw, int G2, int nR, int rows,
+               unsigned long long* __restrict__ wmax) {
+  __shared__ double red[8][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, i = blockIdx.x * 32 + lane;
+  const int g1 = min(G2, (int)(blockIdx.y + 1) * rows);
   double m = 0.0;
-  for (int g = threadIdx.x; g < G2; g += blockDim.x) m = fmax(m, fabs(W[(size_t)g * ldw + i]));
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+  if (i < nR)
+#pragma unroll 8
+    for (int g = blockIdx.y * rows + w; g < g1; g += 8) m = fmax(m, fabs(__ldg(W + (size_t)g * ldw + i)));
+  red[w][lane] = m;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) m = fmax(m, red[w]);
-    m = fmax(m, red[0]);
-    int e = 0;
-    int s = 0;
-    if (m > 0.0) {
-      frexp(m, &e);  // m = f 2^e, f in [0.5, 1)
-      s = 14 - e;
-    }
-    wexp[i] = s;
-    col_scale[i] = ldexp(1.0, -(s + kXScaleExp));
+  if (w == 0 && i < nR) {
+#pragma unroll
+    for (int q = 1; q < 8; ++q) m = fmax(m, red[q][lane]);
+    atomicMax(wmax + i, (unsigned long long)__double_as_longlong(m));
   }
+}
+__device__ __forceinline__ int tc_wexp(unsigned long long bits) {
+  const double m = __longlong_as_double((long long)bits);
+  if (!(m > 0.0)) return 0;
+  int e = 0;
+  frexp(m, &e);  // m = f 2^e, f in [0.5, 1)
+  return 14 - e;
 }
 
 // Column parts of the radial axis: part p covers columns [c0[p], c0[p] + nc[p]).
@@ -240,44 +242,56 @@ struct TcParts {
 // ---------------------------------------------------------------- operand images
 // W (FP64, [g][ldw]) -> per column part p and chunk c: [plane hi/lo][kg 0..7][ng 0..nc/8-1]
 // [8 rows][8 x 16 bit] at part_off(p) + c * 2 * TC_KC * nc(p), part_off(p) = n_chunks * 2 *
-// TC_KC * c0(p); F16x3 scales column n by 2^wexp[n] first (exact).
+// TC_KC * c0(p); F16x3 scales column n by the power of two of tc_wexp first (exact).  A
+// thread takes one column and eight grid points, one 16-byte core-matrix row per plane:
+// reads are coalesced along R, writes along the rows (a thread per value, grid points
+// fastest, read a sector per value).
 template <bool kF16>
-__global__ void tc_bimage_kernel(const double* __restrict__ W, int ldw, int G2, int nR, int npad,
-                                 int n_chunks, TcParts parts, const int* __restrict__ wexp,
-                                 unsigned short* __restrict__ img) {
-  int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  int64_t per_chunk = (int64_t)TC_KC * npad;
-  if (idx >= per_chunk * n_chunks) return;
-  int c = (int)(idx / per_chunk);
-  int rem = (int)(idx % per_chunk);
-  int n = rem / TC_KC, k = rem % TC_KC;
+__global__ void __launch_bounds__(256)
+tc_bimage_kernel(const double* __restrict__ W, int ldw, int G2, int nR, int npad, int n_chunks,
+                 TcParts parts, const unsigned long long* __restrict__ wmax,
+                 double* __restrict__ col_scale, unsigned short* __restrict__ img) {
+  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= (int64_t)npad * 8 * n_chunks) return;
+  const int n = (int)(idx % npad);
+  const int64_t q = idx / npad;
+  const int kg = (int)(q & 7), c = (int)(q >> 3);
   int p = 0;
   while (p + 1 < parts.n && parts.c0[p + 1] <= n) ++p;
   const int nl = n - parts.c0[p], nc = parts.nc[p];
-  int g = c * TC_KC + k;
-  double w = (g < G2 && n < nR) ? W[(size_t)g * ldw + n] : 0.0;
-  unsigned short hi, lo;
-  if (kF16) {
-    if (n < nR) w = ldexp(w, wexp[n]);
-    __half h = __double2half(w);
-    __half l = __double2half(w - (double)__half2float(h));
-    hi = __half_as_ushort(h);
-    lo = __half_as_ushort(l);
-  } else {
-    __nv_bfloat16 h = __double2bfloat16(w);
-    __nv_bfloat16 l = __double2bfloat16(w - (double)__bfloat162float(h));
-    hi = __bfloat16_as_ushort(h);
-    lo = __bfloat16_as_ushort(l);
+  const int g0 = c * TC_KC + kg * 8;
+  const int s = kF16 && n < nR ? tc_wexp(wmax[n]) : 0;
+  if (kF16 && q == 0) col_scale[n] = n < nR ? ldexp(1.0, -(s + kXScaleExp)) : 0.0;
+  double w[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) w[e] = (g0 + e < G2 && n < nR) ? __ldg(W + (size_t)(g0 + e) * ldw + n) : 0.0;
+  unsigned short hi[8], lo[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    if (kF16) {
+      const double x = ldexp(w[e], s);
+      const __half h = __double2half(x);
+      hi[e] = __half_as_ushort(h);
+      lo[e] = __half_as_ushort(__double2half(x - (double)__half2float(h)));
+    } else {
+      const __nv_bfloat16 h = __double2bfloat16(w[e]);
+      hi[e] = __bfloat16_as_ushort(h);
+      lo[e] = __bfloat16_as_ushort(__double2bfloat16(w[e] - (double)__bfloat162float(h)));
+    }
   }
-  int kg = k >> 3, e = k & 7, ng = nl >> 3, r8 = nl & 7;
+  auto pack = [](const unsigned short (&v)[8]) {
+    return make_uint4(v[0] | (unsigned)v[1] << 16, v[2] | (unsigned)v[3] << 16,
+                      v[4] | (unsigned)v[5] << 16, v[6] | (unsigned)v[7] << 16);
+  };
   const size_t plane = (size_t)TC_KC * nc;
   const size_t off = (size_t)n_chunks * 2 * TC_KC * parts.c0[p] + (size_t)c * 2 * plane +
-                     (((size_t)kg * (nc / 8) + ng) * 8 + r8) * 8 + e;
-  img[off] = hi;
-  img[off + plane] = lo;
+                     (((size_t)kg * (nc / 8) + (nl >> 3)) * 8 + (nl & 7)) * 8;
+  *reinterpret_cast<uint4*>(img + off) = pack(hi);
+  *reinterpret_cast<uint4*>(img + off + plane) = pack(lo);
 }
 
-// psi (FP64, [basis row][G2]) -> per (block, chunk): [local state][TC_PSI_LD] float2.
+// psi (FP64, [basis row][G2]) -> per (block, chunk): [local state][TC_PSI_LD] float2, for the
+// bases that are not written as images at once (SYS_TYPE 1).
 __global__ void tc_psiimage_kernel(const double2* __restrict__ psi, int G2, int n_chunks,
                                    const int* __restrict__ blk_row0, const int* __restrict__ blk_n,
                                    const int64_t* __restrict__ blk_img_off, int n_blocks,
@@ -681,11 +695,25 @@ int MatrixPlan::tc_init() {
   MQCT_CUDA_TRY(d_part.alloc((size_t)tc_splits * n_rows * tc_ldp));
   MQCT_CUDA_TRY(d_bimg.alloc((size_t)t.n_chunks * 2 * TC_KC * t.npad));
   MQCT_CUDA_TRY(d_psi32.alloc((size_t)acc));
+  {
+    // (the images' padding, two values a row and the grid points past G2, stays zero)
+    MQCT_CUDA_TRY(cudaMemsetAsync(d_psi32.p, 0, sizeof(float2) * (size_t)acc, stream));
+    std::vector<int64_t> ro(n_basis_rows);
+    std::vector<int> rs(n_basis_rows);
+    for (int b = 0; b < t.n_blocks; ++b)
+      for (int l = 0; l < nb[b]; ++l) {
+        ro[row0[b] + l] = off[b] + (int64_t)l * TC_PSI_LD;
+        rs[row0[b] + l] = nb[b] * TC_PSI_LD;
+      }
+    MQCT_CUDA_TRY(t.row_off.upload(ro, stream));
+    MQCT_CUDA_TRY(t.row_step.upload(rs, stream));
+    MQCT_CUDA_TRY(cudaStreamSynchronize(stream));  // the host arrays end here
+  }
   MQCT_CUDA_TRY(d_status.alloc(1));
   MQCT_CUDA_TRY(cudaMemsetAsync(d_status.p, 0, sizeof(int), stream));
   MQCT_CUDA_TRY(d_col_scale.alloc((size_t)t.npad));
   if (precision == MQCT_PREC_F16X3) {
-    MQCT_CUDA_TRY(t.wexp.alloc((size_t)nR));
+    MQCT_CUDA_TRY(t.wmax.alloc((size_t)nR));
     MQCT_CUDA_TRY(cudaMemsetAsync(d_col_scale.p, 0, sizeof(double) * t.npad, stream));
     MQCT_CUDA_TRY(cudaFuncSetAttribute(tc_contract_kernel<true, 8>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)t.smem));
@@ -712,23 +740,29 @@ int MatrixPlan::tc_execute() {
     parts.c0[p] = t.part_c0[p];
     parts.nc[p] = t.part_nc[p];
   }
-  int64_t nb_img = (int64_t)t.n_chunks * TC_KC * t.npad;
+  const int64_t nb_img = (int64_t)t.n_chunks * 8 * t.npad;
   const unsigned nbb = (unsigned)((nb_img + thr - 1) / thr);
   if (f16) {
-    tc_wscale_kernel<<<(unsigned)nR, 256, 0, stream>>>(d_W.p, ldw, G2, t.wexp.p, d_col_scale.p);
+    MQCT_CUDA_TRY(cudaMemsetAsync(t.wmax.p, 0, sizeof(unsigned long long) * nR, stream));
+    const int nx = (nR + 31) / 32;
+    const int rows = std::max(64, (int)(((int64_t)G2 * nx + 4 * t.n_sm - 1) / (4 * t.n_sm)));
+    tc_wmax_kernel<<<dim3(nx, (G2 + rows - 1) / rows), 256, 0, stream>>>(d_W.p, ldw, G2, nR, rows,
+                                                                         t.wmax.p);
     MQCT_CUDA_TRY(cudaGetLastError());
     tc_bimage_kernel<true><<<nbb, thr, 0, stream>>>(d_W.p, ldw, G2, nR, t.npad, t.n_chunks, parts,
-                                                    t.wexp.p, d_bimg.p);
+                                                    t.wmax.p, d_col_scale.p, d_bimg.p);
   } else {
     tc_bimage_kernel<false><<<nbb, thr, 0, stream>>>(d_W.p, ldw, G2, nR, t.npad, t.n_chunks, parts,
-                                                     nullptr, d_bimg.p);
+                                                     nullptr, nullptr, d_bimg.p);
   }
   MQCT_CUDA_TRY(cudaGetLastError());
-  int64_t np_img = (int64_t)n_basis_rows * t.n_chunks * TC_PSI_LD;
-  tc_psiimage_kernel<<<(unsigned)((np_img + thr - 1) / thr), thr, 0, stream>>>(
-      d_psi.p, G2, t.n_chunks, t.blk_row0.p, t.blk_n.p, t.blk_img_off.p, t.n_blocks, d_psi32.p,
-      n_basis_rows);
-  MQCT_CUDA_TRY(cudaGetLastError());
+  if (sys_type == 1) {
+    const int64_t np_img = (int64_t)n_basis_rows * t.n_chunks * TC_PSI_LD;
+    tc_psiimage_kernel<<<(unsigned)((np_img + thr - 1) / thr), thr, 0, stream>>>(
+        d_psi.p, G2, t.n_chunks, t.blk_row0.p, t.blk_n.p, t.blk_img_off.p, t.n_blocks, d_psi32.p,
+        n_basis_rows);
+    MQCT_CUDA_TRY(cudaGetLastError());
+  }
   TcArgs a{};
   a.n_parts = t.n_parts;
   a.n_ks = tc_splits;

@@ -12,8 +12,8 @@
 // is contracted as written (X recomputed per alpha point).
 //
 // Kernels (one build = K1 + K2 + K3 + K4):
-//   K1 basis_kernel        rotor wavefunctions on the grid, FP64, per m-block
-//   K2 pes_weight_kernel   PES on (grid x R) times the quadrature weights
+//   K1 basis_*_kernel      rotor wavefunctions on the grid, per m-block (basis.cuh)
+//   K2 pes_*_kernel        PES on (grid x R) times the quadrature weights
 //   K3 contract_fp64_kernel / tcgen05 split-precision kernel (contract_tc.cu)
 //   K4 finalize_kernel: FP64 sum of partials, Hartree units, MIJ_CUTOFF,
 //                          clamped spline y2 (one kernel)
@@ -23,6 +23,7 @@
 #include <map>
 #include <mutex>
 
+#include "basis.cuh"
 #include "common.cuh"
 #include "finalize.cuh"
 #include "matrix_plan.cuh"
@@ -93,14 +94,6 @@ __device__ inline double2 asym_wf(int j, int m, const double* c, double alpha, d
   return make_double2(re, im);
 }
 
-// psi for block-local state s at grid point g:
-// type 1: Y_jm(beta, 0) (WF_DIAT_TOP, MQCT_SOURCE_CODES/basis_wave_functions.f:153-175);
-// type 4: sum_K c_K sqrt((2j+1)/8pi^2) d^j_{Km}(beta) e^{iK gamma} at alpha = 0
-//         (WF_ASYM_TOP :83-116 with Djkm MQCT_SOURCE_CODES/pot_comp.f:256-309); the
-//         2-D grid has beta outer, gamma inner;
-// type 0: sum_{m1} CG(j1 m1 j2 m2 | j12 m12) psi1_{m1}(0, beta1, gamma1)
-//         psi2_{m2}(alpha2, beta2, gamma2) (WF_ASYM_TOP_ASYM_TOP :1-41) on the 5-D grid.
-// Output psi[(blk_off + s) * G2 + g] as (re, im) FP64.
 // Rotor tables of the type-4 basis: dtab[(T(j) + (K+j)(2j+1) + (m+j)) * n_beta + ib]
 // = sqrt((2j+1)/8pi^2) d^j_{Km}(beta_ib) with T(j) = sum_{j'<j} (2j'+1)^2, and
 // phase[(K + jmax) * n_gamma + ig] = e^{i K gamma_ig}.  Both depend on the grid
@@ -131,63 +124,70 @@ __global__ void rotor_tables_kernel(int jmax, int n_beta, const double* __restri
   }
 }
 
-template <int SYS>
-__global__ void basis_kernel(int n_rows, const int* __restrict__ row_state,
-                             const int* __restrict__ st_chan, const int* __restrict__ st_m,
-                             const int* __restrict__ ch_j, const double* __restrict__ vec,
-                             int ldv, const double* __restrict__ beta,
-                             const double* __restrict__ gamma, int n_gamma, int G2, Type0Dev t0,
-                             const double* __restrict__ dtab, const double2* __restrict__ phase,
-                             int jmax, double2* __restrict__ psi) {
-  int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (int64_t)n_rows * G2) return;
-  int r = (int)(idx / G2), g2 = (int)(idx % G2);
-  int st = row_state[r];
-  int ch = st_chan[st];
-  int j = ch_j[ch], m = st_m[st];
-  double re = 0.0, im = 0.0;
-  if constexpr (SYS == 1) {
-    double b = beta[g2];
-    int am = m < 0 ? -m : m;
-    double pl = mqct_dev::plgndr(j, am, cos(b));
-    double nrm = sqrt((2.0 * j + 1.0) / 4.0 / kPi * exp(c_logfact[j - am] - c_logfact[j + am]));
-    re = pl * nrm;
-    if (m < 0 && (am & 1)) re = -re;
-  } else if constexpr (SYS == 0) {
-    int ia2, ib1, ib2, ig1, ig2;
-    t0_index(t0, g2, ia2, ib1, ib2, ig1, ig2);
-    const int j2 = t0.ch_j2[ch];
-    const double* c1 = vec + (size_t)ch * ldv;
-    const double* c2 = t0.vec2 + (size_t)ch * ldv;
-    const double* cgs = t0.cg + (size_t)st * t0.cg_ld;
-    for (int m1 = -j; m1 <= j; ++m1) {
-      const int m2 = m - m1;
-      const double w = cgs[m1 + j];
-      if (m2 < -j2 || m2 > j2 || w == 0.0) continue;
-      const double2 p1 = asym_wf(j, m1, c1, 0.0, beta[ib1], gamma[ig1]);
-      const double2 p2 = asym_wf(j2, m2, c2, t0.alpha2[ia2], t0.beta2[ib2], t0.gamma2[ig2]);
-      re += w * (p1.x * p2.x - p1.y * p2.y);
-      im += w * (p1.x * p2.y + p1.y * p2.x);
-    }
-  } else {
-    const int ib = g2 / n_gamma, ig = g2 % n_gamma;
-    const double* c = vec + (size_t)ch * ldv;
-    const int n_beta = G2 / n_gamma;
-    const double* dj = dtab + (size_t)(dtab_off(j) + (m + j)) * n_beta + ib;
-    const double2* pk = phase + (size_t)(jmax - j) * n_gamma + ig;
-    for (int i = 0; i <= 2 * j; ++i) {
-      const double ci = c[i];
-      if (ci == 0.0) continue;
-      const double d = ci * dj[(size_t)i * (2 * j + 1) * n_beta];
-      const double2 e = pk[(size_t)i * n_gamma];
-      re += d * e.x;
-      im += d * e.y;
-    }
+// The per-rotor tables of SYS_TYPE 0 (see PairTab), one thread per entry.
+__global__ void pair_tables_kernel(PairTab t, const int* __restrict__ ch_j1,
+                                   const int* __restrict__ ch_j2, const double* __restrict__ vec1,
+                                   const double* __restrict__ vec2, int ldv, int nb1, int ng1,
+                                   int nbb, int naa, int ngg, const double* __restrict__ beta1,
+                                   const double* __restrict__ gamma1,
+                                   const double* __restrict__ alpha2,
+                                   const double* __restrict__ beta2,
+                                   const double* __restrict__ gamma2) {
+  int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int np1 = nb1 * ng1, np2 = nbb * ngg;
+  if (q < (int64_t)t.n_lm1 * np1) {
+    const int lm = (int)(q / np1), p = (int)(q % np1), ch = t.lm1_ch[lm];
+    t.psi1[q] = asym_wf(ch_j1[ch], t.lm1_m[lm], vec1 + (size_t)ch * ldv, 0.0, beta1[p / ng1],
+                        gamma1[p % ng1]);
+    return;
   }
-  psi[idx] = make_double2(re, im);
+  q -= (int64_t)t.n_lm1 * np1;
+  if (q < (int64_t)t.n_lm2 * np2) {
+    const int lm = (int)(q / np2), p = (int)(q % np2), ch = t.lm2_ch[lm];
+    t.psi2[q] = asym_wf(ch_j2[ch], t.lm2_m[lm], vec2 + (size_t)ch * ldv, 0.0, beta2[p / ngg],
+                        gamma2[p % ngg]);
+    return;
+  }
+  q -= (int64_t)t.n_lm2 * np2;
+  if (q < (int64_t)(2 * t.J2 + 1) * naa) {
+    double sn, co;
+    sincos((double)((int)(q / naa) - t.J2) * alpha2[q % naa], &sn, &co);
+    t.ph2[q] = make_double2(co, sn);
+    return;
+  }
+  q -= (int64_t)(2 * t.J2 + 1) * naa;
+  if (q < (int64_t)np1 * t.n_s1) {
+    const int p = (int)(q / t.n_s1), s = (int)(q % t.n_s1);
+    euler_apply(0.0, beta1[p / ng1], gamma1[p % ng1], t.s1 + 3 * s, t.x1 + 3 * q);
+    return;
+  }
+  q -= (int64_t)np1 * t.n_s1;
+  if (q < (int64_t)naa * np2 * t.n_s2) {
+    const int s = (int)(q % t.n_s2), p = (int)(q / t.n_s2), ig2 = p % ngg, r = p / ngg;
+    euler_apply(alpha2[r / nbb], beta2[r % nbb], gamma2[ig2], t.s2 + 3 * s, t.x2 + 3 * q);
+  }
+}
+
+// psi of the diatom, SYS_TYPE 1: Y_jm(beta, 0) (WF_DIAT_TOP,
+// MQCT_SOURCE_CODES/basis_wave_functions.f:153-175), psi[row * G2 + g] FP64.
+__global__ void basis_diatom_kernel(int n_rows, const int* __restrict__ row_state,
+                                    const int* __restrict__ st_chan, const int* __restrict__ st_m,
+                                    const int* __restrict__ ch_j, const double* __restrict__ beta,
+                                    int G2, double2* __restrict__ psi) {
+  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= (int64_t)n_rows * G2) return;
+  const int r = (int)(idx / G2), g2 = (int)(idx % G2);
+  const int st = row_state[r], j = ch_j[st_chan[st]], m = st_m[st], am = m < 0 ? -m : m;
+  const double pl = mqct_dev::plgndr(j, am, cos(beta[g2]));
+  const double nrm = sqrt((2.0 * j + 1.0) / 4.0 / kPi * exp(c_logfact[j - am] - c_logfact[j + am]));
+  double re = pl * nrm;
+  if (m < 0 && (am & 1)) re = -re;
+  psi[idx] = make_double2(re, 0.0);
 }
 
 // ------------------------------------------------------------------ K2: PES x weights
+// Site surfaces and the Legendre surface have kernels of their own (basis.cuh); this one
+// serves tables and surfaces beyond their limits.
 // W[g2 * ldw + i] = wt[g2] * V(R_i, angles(g2)) with the argument mapping of
 // MQCT_SOURCE_CODES/pes_sys_type.f: type 1 passes beta (:8), type 4 passes
 // (-beta, -gamma) (:36), type 0 passes (0, beta1, gamma1, alpha2, beta2, gamma2)
@@ -869,6 +869,42 @@ int MatrixPlan::init(const mqct_sys_t* sys, const int32_t* ind_mat, int64_t P_, 
         cg[(size_t)st * cg_ld + m1 + j1] =
             clebsch_gordan(j1, m1, j2, sys->m12[st] - m1, sys->j12[st], sys->m12[st]);
     }
+    // the distinct levels (j, vector) of each rotor and their (level, m) tables
+    auto levels = [&](const int32_t* j, const double* v, std::vector<int>& lm_ch,
+                      std::vector<int>& lm_m, std::vector<int>& ch_lm) {
+      std::vector<int> rep, first;  // a channel per level, the place of its (level, -j)
+      ch_lm.resize(sys->n_channels);
+      for (int c = 0; c < sys->n_channels; ++c) {
+        const double* vc = v + (size_t)c * ldv;
+        size_t l = 0;
+        while (l < rep.size() && !(j[rep[l]] == j[c] &&
+                                   std::equal(vc, vc + 2 * j[c] + 1, v + (size_t)rep[l] * ldv)))
+          ++l;
+        if (l == rep.size()) {
+          rep.push_back(c);
+          first.push_back((int)lm_ch.size());
+          for (int m = -j[c]; m <= j[c]; ++m) {
+            lm_ch.push_back(c);
+            lm_m.push_back(m);
+          }
+        }
+        ch_lm[c] = first[l];
+      }
+    };
+    std::vector<int> lc[2], lm[2], cl[2];
+    levels(sys->j1, sys->vec1, lc[0], lm[0], cl[0]);
+    levels(sys->j2, sys->vec2, lc[1], lm[1], cl[1]);
+    for (int r = 0; r < 2; ++r) {
+      t0_n_lm[r] = (int)lc[r].size();
+      MQCT_CUDA_TRY(d_lm_ch[r].upload(lc[r], stream));
+      MQCT_CUDA_TRY(d_lm_m[r].upload(lm[r], stream));
+      MQCT_CUDA_TRY(d_ch_lm[r].upload(cl[r], stream));
+    }
+    t0_J2 = 0;
+    for (int c = 0; c < sys->n_channels; ++c) t0_J2 = std::max(t0_J2, (int)sys->j2[c]);
+    MQCT_CUDA_TRY(d_pair_psi.alloc((size_t)t0_n_lm[0] * grid->n_beta * n_gamma +
+                                   (size_t)t0_n_lm[1] * t0_nbb * t0_ngg +
+                                   (size_t)(2 * t0_J2 + 1) * t0_naa));
     MQCT_CUDA_TRY(d_ch_j2.upload(ch_j2, stream));
     MQCT_CUDA_TRY(d_cg.upload(cg, stream));
     MQCT_CUDA_TRY(d_vec2.upload(sys->vec2, (size_t)sys->n_channels * ldv, stream));
@@ -923,10 +959,18 @@ int MatrixPlan::init(const mqct_sys_t* sys, const int32_t* ind_mat, int64_t P_, 
     }
   }
 
+  rc = upload_site_terms(pes);
+  if (rc) return rc;
+  if (sys_type == 0 && pes_sites)
+    MQCT_CUDA_TRY(d_pair_x.alloc(3 * ((size_t)grid->n_beta * n_gamma * pes_n_sites1 +
+                                      (size_t)t0_naa * t0_nbb * t0_ngg * pes_n_sites2)));
+
   // --- grid-only coefficients of the fused spline fit (finalize_kernel)
   MQCT_CUDA_TRY(d_spl_fin.upload(spline_grid_coefs(Rh), stream));
   // --- work buffers
-  MQCT_CUDA_TRY(d_psi.alloc((size_t)n_basis_rows * G2));
+  // (the tensor-core form of rotor bases is written as FP32 images, tc_init)
+  if (precision == MQCT_PREC_FP64 || sys_type == 1)
+    MQCT_CUDA_TRY(d_psi.alloc((size_t)n_basis_rows * G2));
   ldw = nR;
   MQCT_CUDA_TRY(d_W.alloc((size_t)G2 * ldw));
   if (precision == MQCT_PREC_FP64) {
@@ -941,48 +985,141 @@ int MatrixPlan::init(const mqct_sys_t* sys, const int32_t* ind_mat, int64_t P_, 
   return MQCT_OK;
 }
 
-int MatrixPlan::run_basis_and_pes() {
-  int threads = 256;
-  int64_t nb = (int64_t)n_basis_rows * G2;
-  const Type0Dev t0{d_ch_j2.p, d_vec2.p, d_cg.p, cg_ld, d_beta2.p, d_alpha2.p, d_gamma2.p,
-                    (int)h_beta.size(), n_gamma, t0_nbb, t0_naa, t0_ngg};
-  const unsigned gb = (unsigned)((nb + threads - 1) / threads);
-  if (sys_type == 4) {
-    const int n_tab = dtab_off(jmax_basis + 1) * (int)h_beta.size() + (2 * jmax_basis + 1) * n_gamma;
-    rotor_tables_kernel<<<(unsigned)((n_tab + threads - 1) / threads), threads, 0, stream>>>(
-        jmax_basis, (int)h_beta.size(), d_beta.p, n_gamma, d_gamma.p, d_dtab.p, d_phase.p);
-    MQCT_CUDA_TRY(cudaGetLastError());
+// The PES's site terms in the order of their distinct sites (SiteTerms); pes_sites tells
+// whether the surface has that form.
+int MatrixPlan::upload_site_terms(const mqct_pes_t* pes) {
+  pes_sites = false;
+  if (pes->kind != MQCT_PES_SITES1 && pes->kind != MQCT_PES_SITES2) return MQCT_OK;
+  const bool two = pes->kind == MQCT_PES_SITES2;
+  const int per = two ? 7 : 6, nt = pes->n_terms;
+  if (nt > kSiteMax) return MQCT_OK;
+  std::vector<std::pair<int, int>> us;
+  std::vector<std::vector<int>> terms;
+  for (int t = 0; t < nt; ++t) {
+    const std::pair<int, int> k((int)pes->params[per * t], two ? (int)pes->params[per * t + 1] : 0);
+    const size_t u = std::find(us.begin(), us.end(), k) - us.begin();
+    if (u == us.size()) {
+      us.push_back(k);
+      terms.emplace_back();
+    }
+    terms[u].push_back(t);
   }
-  if (sys_type == 1)
-    basis_kernel<1><<<gb, threads, 0, stream>>>(n_basis_rows, d_row_state.p, d_st_chan.p,
-                                                d_st_m.p, d_ch_j.p, d_vec.p, ldv, d_beta.p,
-                                                d_gamma.p, n_gamma, G2, t0, d_dtab.p, d_phase.p,
-                                                jmax_basis, d_psi.p);
-  else if (sys_type == 4)
-    basis_kernel<4><<<gb, threads, 0, stream>>>(n_basis_rows, d_row_state.p, d_st_chan.p,
-                                                d_st_m.p, d_ch_j.p, d_vec.p, ldv, d_beta.p,
-                                                d_gamma.p, n_gamma, G2, t0, d_dtab.p, d_phase.p,
-                                                jmax_basis, d_psi.p);
-  else
-    basis_kernel<0><<<gb, threads, 0, stream>>>(n_basis_rows, d_row_state.p, d_st_chan.p,
-                                                d_st_m.p, d_ch_j.p, d_vec.p, ldv, d_beta.p,
-                                                d_gamma.p, n_gamma, G2, t0, d_dtab.p, d_phase.p,
-                                                jmax_basis, d_psi.p);
+  std::vector<int> u0(1, 0), us1, us2;
+  std::vector<double> q;
+  for (size_t u = 0; u < us.size(); ++u) {
+    us1.push_back(us[u].first);
+    us2.push_back(us[u].second);
+    for (int t : terms[u]) {
+      const double* p = pes->params + (size_t)per * t + (two ? 2 : 1);  // D, a, re, C6, rd
+      q.insert(q.end(), {p[1], p[2], p[0], p[3], 1.0 / (p[4] * p[4])});
+    }
+    u0.push_back((int)q.size() / 5);
+  }
+  site_n_u = (int)us.size();
+  const size_t ni = u0.size() + us1.size() + us2.size();
+  if (d_site_i.n != ni) MQCT_CUDA_TRY(d_site_i.alloc(ni));
+  if (d_site_q.n != q.size()) MQCT_CUDA_TRY(d_site_q.alloc(q.size()));
+  MQCT_CUDA_TRY(cudaMemcpyAsync(d_site_q.p, q.data(), sizeof(double) * q.size(),
+                                cudaMemcpyHostToDevice, stream));
+  u0.insert(u0.end(), us1.begin(), us1.end());
+  u0.insert(u0.end(), us2.begin(), us2.end());
+  MQCT_CUDA_TRY(cudaMemcpyAsync(d_site_i.p, u0.data(), sizeof(int) * u0.size(),
+                                cudaMemcpyHostToDevice, stream));
+  MQCT_CUDA_TRY(cudaStreamSynchronize(stream));  // the host arrays end here
+  pes_sites = true;
+  return MQCT_OK;
+}
+
+int MatrixPlan::run_basis_and_pes() {
+  const int threads = 256;
+  const int n_beta = (int)h_beta.size();
+  const Type0Dev t0{d_ch_j2.p, d_vec2.p, d_cg.p, cg_ld, d_beta2.p, d_alpha2.p, d_gamma2.p,
+                    n_beta, n_gamma, t0_nbb, t0_naa, t0_ngg};
+  const bool img = precision != MQCT_PREC_FP64;
+  const BasisOut out{d_psi.p, d_psi32.p, tc ? tc->row_off.p : nullptr, tc ? tc->row_step.p : nullptr,
+                     G2};
+  PairTab pt{};
+  if (sys_type == 4) {
+    const int n_tab = dtab_off(jmax_basis + 1) * n_beta + (2 * jmax_basis + 1) * n_gamma;
+    rotor_tables_kernel<<<(unsigned)((n_tab + threads - 1) / threads), threads, 0, stream>>>(
+        jmax_basis, n_beta, d_beta.p, n_gamma, d_gamma.p, d_dtab.p, d_phase.p);
+    MQCT_CUDA_TRY(cudaGetLastError());
+    (img ? basis_top_kernel<true> : basis_top_kernel<false>)<<<(unsigned)n_basis_rows, threads, 0,
+                                                              stream>>>(
+        d_row_state.p, d_st_chan.p, d_st_m.p, d_ch_j.p, d_vec.p, ldv, n_beta, n_gamma, d_dtab.p,
+        d_phase.p, jmax_basis, out);
+  } else if (sys_type == 1) {
+    const int64_t nb = (int64_t)n_basis_rows * G2;
+    basis_diatom_kernel<<<(unsigned)((nb + threads - 1) / threads), threads, 0, stream>>>(
+        n_basis_rows, d_row_state.p, d_st_chan.p, d_st_m.p, d_ch_j.p, d_beta.p, G2, d_psi.p);
+  } else {
+    const int64_t np1 = (int64_t)n_beta * n_gamma, np2 = (int64_t)t0_nbb * t0_ngg;
+    pt.n_lm1 = t0_n_lm[0];
+    pt.n_lm2 = t0_n_lm[1];
+    pt.lm1_ch = d_lm_ch[0].p;
+    pt.lm1_m = d_lm_m[0].p;
+    pt.lm2_ch = d_lm_ch[1].p;
+    pt.lm2_m = d_lm_m[1].p;
+    pt.ch_lm1 = d_ch_lm[0].p;
+    pt.ch_lm2 = d_ch_lm[1].p;
+    pt.J2 = t0_J2;
+    pt.n_s1 = pes_sites ? pes_n_sites1 : 0;
+    pt.n_s2 = pes_sites ? pes_n_sites2 : 0;
+    pt.s1 = d_pes_s1.p;
+    pt.s2 = d_pes_s2.p;
+    pt.psi1 = d_pair_psi.p;
+    pt.psi2 = pt.psi1 + pt.n_lm1 * np1;
+    pt.ph2 = pt.psi2 + pt.n_lm2 * np2;
+    pt.x1 = d_pair_x.p;
+    pt.x2 = pt.x1 + 3 * np1 * pt.n_s1;
+    const int64_t n_tab = pt.n_lm1 * np1 + pt.n_lm2 * np2 + (int64_t)(2 * t0_J2 + 1) * t0_naa +
+                          np1 * pt.n_s1 + t0_naa * np2 * pt.n_s2;
+    pair_tables_kernel<<<(unsigned)((n_tab + 127) / 128), 128, 0, stream>>>(
+        pt, d_ch_j.p, d_ch_j2.p, d_vec.p, d_vec2.p, ldv, n_beta, n_gamma, t0_nbb, t0_naa, t0_ngg,
+        d_beta.p, d_gamma.p, d_alpha2.p, d_beta2.p, d_gamma2.p);
+    MQCT_CUDA_TRY(cudaGetLastError());
+    const dim3 gr((unsigned)((G2 + threads - 1) / threads),
+                  (unsigned)((n_basis_rows + kRowRun - 1) / kRowRun));
+    (img ? basis_pair_kernel<true> : basis_pair_kernel<false>)<<<gr, threads, 0, stream>>>(
+        n_basis_rows, d_row_state.p, d_st_chan.p, d_st_m.p, d_ch_j.p, d_ch_j2.p, d_cg.p, cg_ld,
+        n_beta, n_gamma, t0_nbb, t0_naa, t0_ngg, pt, out);
+  }
   MQCT_CUDA_TRY(cudaGetLastError());
   PesDev pd{pes_kind, pes_n_terms, pes_n_sites1, pes_n_sites2, d_pes_p.p, d_pes_s1.p, d_pes_s2.p,
             d_pes_table.p};
-  int64_t nw = (int64_t)G2 * nR;
-  const unsigned gw = (unsigned)((nw + threads - 1) / threads);
   if (sur) return run_surrogate_pes(pd, t0);
-  if (sys_type == 1)
-    pes_weight_kernel<1><<<gw, threads, 0, stream>>>(pd, G2, nR, d_R.p, d_beta.p, d_gamma.p,
-                                                     n_gamma, t0, d_wt.p, d_W.p, ldw);
-  else if (sys_type == 4)
-    pes_weight_kernel<4><<<gw, threads, 0, stream>>>(pd, G2, nR, d_R.p, d_beta.p, d_gamma.p,
-                                                     n_gamma, t0, d_wt.p, d_W.p, ldw);
-  else
-    pes_weight_kernel<0><<<gw, threads, 0, stream>>>(pd, G2, nR, d_R.p, d_beta.p, d_gamma.p,
-                                                     n_gamma, t0, d_wt.p, d_W.p, ldw);
+  if (pes_sites) {
+    const SiteTerms ps{pes_n_terms, site_n_u, d_site_i.p, d_site_i.p + site_n_u + 1,
+                       d_site_i.p + 2 * site_n_u + 1, d_site_q.p};
+    // grid points per CTA: sixteen (the items of a CTA then fill its rounds to a few percent),
+    // fewer where the grid is small (four CTAs per SM) or the sites are many
+    const int GB = std::max(1, std::min({16, kGeoMax / site_n_u, G2 / (4 * n_sm)}));
+    const unsigned gr = (unsigned)((G2 + GB - 1) / GB);
+    const size_t sm = sizeof(double) * 5 * (size_t)pes_n_terms + sizeof(int) * (size_t)(site_n_u + 1);
+    auto go = [&](auto kern) {
+      kern<<<gr, 128, sm, stream>>>(ps, G2, nR, GB, d_R.p, d_beta.p, d_gamma.p, n_gamma, d_pes_s1.p,
+                                    n_beta, n_gamma, t0_nbb, t0_ngg, pes_n_sites1, pes_n_sites2,
+                                    pt.x1, pt.x2, d_wt.p, d_W.p, ldw);
+    };
+    if (sys_type == 1) go(pes_sites_kernel<1>);
+    else if (sys_type == 4) go(pes_sites_kernel<4>);
+    else go(pes_sites_kernel<0>);
+  } else if (pes_kind == MQCT_PES_LEGENDRE && pes_n_terms <= kLegMax &&
+             (G2 + kLegG - 1) / kLegG <= 65535) {
+    const dim3 gr((unsigned)((nR + 127) / 128), (unsigned)((G2 + kLegG - 1) / kLegG));
+    pes_legendre_kernel<<<gr, 128, 0, stream>>>(pes_n_terms, d_pes_p.p, G2, nR, d_R.p, d_beta.p,
+                                                n_gamma, d_wt.p, d_W.p, ldw);
+  } else {
+    const int64_t nw = (int64_t)G2 * nR;
+    const unsigned gw = (unsigned)((nw + threads - 1) / threads);
+    auto go = [&](auto kern) {
+      kern<<<gw, threads, 0, stream>>>(pd, G2, nR, d_R.p, d_beta.p, d_gamma.p, n_gamma, t0, d_wt.p,
+                                       d_W.p, ldw);
+    };
+    if (sys_type == 1) go(pes_weight_kernel<1>);
+    else if (sys_type == 4) go(pes_weight_kernel<4>);
+    else go(pes_weight_kernel<0>);
+  }
   MQCT_CUDA_TRY(cudaGetLastError());
   return MQCT_OK;
 }
@@ -1074,7 +1211,7 @@ int MatrixPlan::refresh_inputs(const mqct_sys_t* sys, const double* R, const mqc
       MQCT_CUDA_TRY(cudaMemcpyAsync(d_pes_s2.p, pes->sites2, sizeof(double) * d_pes_s2.n,
                                     cudaMemcpyHostToDevice, stream));
   }
-  return MQCT_OK;
+  return upload_site_terms(pes);
 }
 
 double MatrixPlan::flops() const {

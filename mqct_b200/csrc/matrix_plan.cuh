@@ -36,7 +36,9 @@ struct TcInfo {
   DevBuf<int> blk_row0, blk_n, blk_m;
   DevBuf<int64_t> blk_img_off;
   DevBuf<double> walpha;
-  DevBuf<int> wexp;  // F16x3: power-of-two exponent of each W column
+  DevBuf<unsigned long long> wmax;  // F16x3: bits of max |W| of each column
+  DevBuf<int64_t> row_off;  // per basis row: its place in the image of chunk 0
+  DevBuf<int> row_step;     // and the distance to its place in the next chunk
 };
 
 struct MatrixPlan {
@@ -72,6 +74,17 @@ struct MatrixPlan {
   DevBuf<int> d_ch_j2;
   DevBuf<double> d_vec2, d_cg, d_beta2, d_alpha2, d_gamma2;
   int cg_ld = 1, t0_nbb = 1, t0_naa = 1, t0_ngg = 1;
+  // its per-rotor tables (rebuilt by every execute): (level, m) lists, wavefunctions with the
+  // alpha2 phases, rotated sites
+  int t0_n_lm[2] = {0, 0}, t0_J2 = 0;
+  DevBuf<int> d_lm_ch[2], d_lm_m[2], d_ch_lm[2];
+  DevBuf<double2> d_pair_psi;
+  DevBuf<double> d_pair_x;
+  // site surface by its distinct sites (SiteTerms): u0, us1, us2 in one array
+  bool pes_sites = false;
+  int site_n_u = 0;
+  DevBuf<int> d_site_i;
+  DevBuf<double> d_site_q;
   // type 4: rotor d-function and gamma-phase tables (rebuilt by every execute)
   DevBuf<double> d_dtab;
   DevBuf<double2> d_phase;
@@ -85,7 +98,7 @@ struct MatrixPlan {
   DevBuf<unsigned> d_sur_ratio;
 
   // work
-  DevBuf<double2> d_psi;  // basis rows x G2, FP64
+  DevBuf<double2> d_psi;  // basis rows x G2, FP64 (FP64 form, and SYS_TYPE 1)
   DevBuf<double> d_W;     // G2 x ldw, FP64
   int ldw = 0;
   DevBuf<double> d_acc;   // FP64 form: n_rows x nR
@@ -108,6 +121,7 @@ struct MatrixPlan {
            const mqct_grid_t* grid, const mqct_pes_t* pes, int32_t prec, double mij_cut,
            double rc1, double rc2);
   int refresh_inputs(const mqct_sys_t* sys, const double* R, const mqct_pes_t* pes);
+  int upload_site_terms(const mqct_pes_t* pes);
   int run_basis_and_pes();
   int run_surrogate_pes(const struct PesDev& pd, const struct Type0Dev& t0);
   int execute(double* d_mat, double* d_y2, int32_t* d_skipped);
