@@ -304,14 +304,27 @@ __global__ void sur_weight_kernel(PesDev pes, int G2, int nR, const double* __re
 
 // ------------------------------------------------------------------ K3: FP64 form
 // acc[row, i] = sum_alpha w_alpha sum_g2 Re(psi_a^* psi_b)[row, g2] W[g2, i] on the FP64
-// tensor cores (mma.sync m8n8k4 f64): a 128 x 64 tile per CTA, 256 threads, K-chunks of
+// tensor cores (mma.sync m8n8k4 f64): a 128 x 8 NT WC tile per CTA of 4 WC warps, K-chunks of
 // 16 grid points.  The integrand of a same-m pair at an alpha point is w_alpha times the
-// alpha-free product (the e^{i m alpha} phases of the two states cancel); it is formed
-// once per chunk and every alpha point is contracted.  Warp w takes rows 32 (w % 4) ..
-// +31 and columns 32 (w / 4) .. +31: 4 x 4 MMA tiles of 8 x 8, 32 FP64 accumulators
-// per lane.  Fixed summation order: reproducible.
-constexpr int F_TM = 128, F_TN = 64, F_TK = 16;
-constexpr int F_XLD = F_TM + 8, F_WLD = F_TN + 8;  // padded rows: 2 wavefronts per fragment load
+// alpha-free product (the e^{i m alpha} phases of the two states cancel); every alpha point
+// is contracted, as a chunk of its own.  Warp w takes rows 32 (w % 4) .. +31 and 8 NT columns
+// from 8 NT (w / 4): 4 x NT MMA tiles of 8 x 8, 8 NT FP64 accumulators per lane.  Fixed
+// summation order: reproducible.
+// What bounds it: the FP64 tensor pipe, as long as forming X keeps out of its way.  The
+// earlier 128 x 64 tile formed X from loads that touched 32 cache lines each, between two
+// barriers with the MMA pipe idle: 3 445 us at 33 280 rows x 2 304 points x 300 R (0.33 of the
+// FP64 rate).  Here sixteen lanes read the 16 grid points of one row (four lines a load), the
+// next chunk's products are loaded and formed between the MMAs of this one, into the other of
+// two shared buffers, W arrives by cp.async, and two CTAs of eight warps share an SM: 2 115
+// us.  The pipe is then what the warps wait for, at 0.66 of its nominal rate; m16n8k8 (2 160
+// us), one CTA of sixteen warps on 160 columns (2 217 us) and plain FMAs on 8 x 10 register
+// tiles (3 066 us) were no faster.
+constexpr int F_TM = 128, F_TK = 16;
+constexpr int F_XLD = F_TK + 4;  // 4 mod 16: an A fragment's 4 rows x 4 points in distinct banks
+__host__ __device__ constexpr int f_wld(int TN) { return (TN + 15) / 16 * 16 + 4; }
+__host__ __device__ constexpr size_t f_smem(int TN) {
+  return sizeof(double) * 2 * (F_TM * F_XLD + F_TK * f_wld(TN));
+}
 // D (8x8) += A (8x4, row) * B (4x8, col) in FP64: lane l holds A[l/4][l%4], B[l%4][l/4] and
 // D[l/4][2 (l%4)], D[l/4][2 (l%4) + 1].
 __device__ __forceinline__ void dmma_884(double& d0, double& d1, double a, double b) {
@@ -319,81 +332,149 @@ __device__ __forceinline__ void dmma_884(double& d0, double& d1, double a, doubl
                : "+d"(d0), "+d"(d1)
                : "d"(a), "d"(b));
 }
-__global__ void __launch_bounds__(256)
-contract_fp64_kernel(int n_rows, int G2, int nR, const int* __restrict__ row_a,
-                     const int* __restrict__ row_b, const double2* __restrict__ psi,
-                     const double* __restrict__ W, int ldw, int n_alpha,
-                     const double* __restrict__ walpha, double* __restrict__ acc) {
-  __shared__ double Xs[F_TK][F_XLD];
-  __shared__ double Ws[F_TK][F_WLD];
+template <int NT, int WC>
+__global__ void __launch_bounds__(128 * WC, 4 / WC)
+contract_fp64_kernel(int G2, int nR, const int* __restrict__ row_a, const int* __restrict__ row_b,
+                     const double2* __restrict__ psi, const double* __restrict__ W, int ldw,
+                     int n_alpha, const double* __restrict__ walpha, double* __restrict__ acc) {
+  constexpr int TN = 8 * NT * WC, WLD = f_wld(TN), THREADS = 128 * WC;
+  constexpr int NX = 4 / WC;                       // X row pairs of a warp formed per k-step
+  extern __shared__ double f_sm[];
+  double* Xs = f_sm;                               // 2 x F_TM x F_XLD
+  double* Ws = f_sm + 2 * F_TM * F_XLD;            // 2 x F_TK x WLD
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int row0 = blockIdx.x * F_TM, col0 = blockIdx.y * F_TN;
-  const int wr = (warp & 3) * 32, wc = (warp >> 2) * 32;
+  const int row0 = blockIdx.x * F_TM, col0 = blockIdx.y * TN;
+  const int wr = (warp & 3) * 32, wc = (warp >> 2) * 8 * NT;
   const int gq = lane >> 2, tq = lane & 3;
-  double c[4][4][2];
+  double c[4][NT][2];
 #pragma unroll
   for (int a = 0; a < 4; ++a)
 #pragma unroll
-    for (int b = 0; b < 4; ++b) c[a][b][0] = c[a][b][1] = 0.0;
-  // X generation: thread -> row tid / 2, grid points 8 (tid % 2) .. +7 of the chunk
-  const int xr = tid >> 1, xg0 = (tid & 1) * 8;
-  const int grow = row0 + xr;
-  const double2* pa = nullptr;
-  const double2* pb = nullptr;
-  if (grow < n_rows) {
-    pa = psi + (size_t)row_a[grow] * G2;
-    pb = psi + (size_t)row_b[grow] * G2;
-  }
+    for (int b = 0; b < NT; ++b) c[a][b][0] = c[a][b][1] = 0.0;
+  // X: a warp forms 8 NX rows, two at a time, a lane per grid point, NX pairs of rows in each
+  // k-step (the rows are padded to whole tiles)
+  const int xk = lane & 15, xr = warp * 8 * NX + (lane >> 4);
+  const int* pra = row_a + row0 + xr;
+  const int* prb = row_b + row0 + xr;
   const int na = n_alpha > 0 ? n_alpha : 1;
-  for (int k0 = 0; k0 < G2; k0 += F_TK) {
+  const int n_vc = (G2 + F_TK - 1) / F_TK * na;    // chunks, each alpha point its own
+  auto load_w = [&](int ck, int buf) {
+    for (int q = tid; q < F_TK * TN; q += THREADS) {
+      const int kk = q / TN, cc = q - kk * TN, g = ck * F_TK + kk, col = col0 + cc;
+      const bool in = g < G2 && col < nR;
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(
+                       (uint32_t)__cvta_generic_to_shared(Ws + (buf * F_TK + kk) * WLD + cc)),
+                   "l"(W + (in ? (size_t)g * ldw + col : 0)), "r"(in ? 8 : 0)
+                   : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  double2 u[NX], v[NX];
+  auto load_x = [&](int ck, int h) {
+    const int g = ck * F_TK + xk;
+#pragma unroll
+    for (int q = 0; q < NX; ++q) {
+      u[q] = v[q] = make_double2(0.0, 0.0);
+      if (g < G2) {
+        u[q] = __ldg(psi + (size_t)__ldg(pra + 2 * (NX * h + q)) * G2 + g);
+        v[q] = __ldg(psi + (size_t)__ldg(prb + 2 * (NX * h + q)) * G2 + g);
+      }
+    }
+  };
+  auto form_x = [&](double wa, int h, int buf) {
+#pragma unroll
+    for (int q = 0; q < NX; ++q)
+      Xs[(buf * F_TM + xr + 2 * (NX * h + q)) * F_XLD + xk] = wa * (u[q].x * v[q].x + u[q].y * v[q].y);
+  };
+  auto weight = [&](int al) { return n_alpha > 0 ? __ldg(walpha + al) : 1.0; };
+  auto mma = [&](int ks, int buf) {
+    double av[4], bv[NT];
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+      av[a] = Xs[(buf * F_TM + wr + 8 * a + gq) * F_XLD + 4 * ks + tq];
+#pragma unroll
+    for (int b = 0; b < NT; ++b) bv[b] = Ws[(buf * F_TK + 4 * ks + tq) * WLD + wc + 8 * b + gq];
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int b = 0; b < NT; ++b) dmma_884(c[a][b][0], c[a][b][1], av[a], bv[b]);
+  };
+  load_w(0, 0);
+  {
+    const double wa = weight(0);
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      load_x(0, h);
+      form_x(wa, h, 0);
+    }
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  int ck = 0, al = 0;
+  for (int vc = 0; vc < n_vc; ++vc) {
+    const int cur = vc & 1, nxt = cur ^ 1;
+    const bool more = vc + 1 < n_vc;
+    if (++al == na) {
+      al = 0;
+      ++ck;
+    }
+    double wa = 1.0;
+    if (more) {
+      load_w(ck, nxt);
+      wa = weight(al);
+    }
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      if (more) load_x(ck, h);
+      mma(h, cur);
+      if (more) form_x(wa, h, nxt);
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
-    for (int q = tid; q < F_TK * F_TN; q += 256) {
-      const int kk = q / F_TN, cc = q % F_TN;
-      const int g = k0 + kk, col = col0 + cc;
-      Ws[kk][cc] = (g < G2 && col < nR) ? W[(size_t)g * ldw + col] : 0.0;
-    }
-    double x[8];
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const int g = k0 + xg0 + e;
-      x[e] = 0.0;
-      if (pa && g < G2) {
-        const double2 u = pa[g], v = pb[g];
-        x[e] = u.x * v.x + u.y * v.y;
-      }
-    }
-    for (int al = 0; al < na; ++al) {
-      const double wa = n_alpha > 0 ? walpha[al] : 1.0;
-      if (al > 0) __syncthreads();  // the previous alpha point's MMAs have read Xs
-#pragma unroll
-      for (int e = 0; e < 8; ++e) Xs[xg0 + e][xr] = wa * x[e];
-      __syncthreads();
-#pragma unroll
-      for (int ks = 0; ks < F_TK / 4; ++ks) {
-        double av[4], bv[4];
-#pragma unroll
-        for (int a = 0; a < 4; ++a) av[a] = Xs[4 * ks + tq][wr + 8 * a + gq];
-#pragma unroll
-        for (int b = 0; b < 4; ++b) bv[b] = Ws[4 * ks + tq][wc + 8 * b + gq];
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-          for (int b = 0; b < 4; ++b) dmma_884(c[a][b][0], c[a][b][1], av[a], bv[b]);
-      }
-    }
   }
 #pragma unroll
   for (int a = 0; a < 4; ++a) {
-    const int row = row0 + wr + 8 * a + gq;
-    if (row >= n_rows) continue;
+    double* out = acc + (size_t)(row0 + wr + 8 * a + gq) * nR;
 #pragma unroll
-    for (int b = 0; b < 4; ++b)
+    for (int b = 0; b < NT; ++b)
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
         const int col = col0 + wc + 8 * b + 2 * tq + i;
-        if (col < nR) acc[(size_t)row * nR + col] = c[a][b][i];
+        if (col < nR) out[col] = c[a][b][i];
       }
   }
+}
+
+// Tile shapes: (NT, WC) with the clocks of one chunk measured on a B200 with the SM's places
+// (4 / WC CTAs) filled; the shape with the least waves x clocks is taken.  The wide shapes
+// win where there are many tiles (2 115 us for 260 row tiles x 300 R against 2 480 with 32
+// columns), 32 columns by sixteen warps where a build has too few tiles to fill the GPU (19
+// row tiles x 201 R x 576 points: 53 us against 80 with 64 columns; before 146).
+struct FpShape {
+  int nt, wc, clocks;
+  const void* fn;
+};
+static const FpShape kFpShapes[] = {
+    {1, 4, 2900, (const void*)contract_fp64_kernel<1, 4>},
+    {2, 2, 3770, (const void*)contract_fp64_kernel<2, 2>},
+    {3, 2, 4980, (const void*)contract_fp64_kernel<3, 2>},
+    {4, 2, 5770, (const void*)contract_fp64_kernel<4, 2>},
+    {5, 2, 7580, (const void*)contract_fp64_kernel<5, 2>},
+};
+static int contract_fp64_shape(int n_tiles, int nR, int n_sm) {
+  int best = 0;
+  double cost = 0.0;
+  for (int q = 0; q < (int)(sizeof kFpShapes / sizeof kFpShapes[0]); ++q) {
+    const FpShape& f = kFpShapes[q];
+    const int tn = 8 * f.nt * f.wc;
+    const int64_t units = (int64_t)n_tiles * ((nR + tn - 1) / tn), places = (int64_t)n_sm * 4 / f.wc;
+    const double t = (double)((units + places - 1) / places) * f.clocks;
+    if (q == 0 || t < cost) {
+      best = q;
+      cost = t;
+    }
+  }
+  return best;
 }
 
 // ------------------------------------------------------------------ K4: finalize
@@ -975,6 +1056,10 @@ int MatrixPlan::init(const mqct_sys_t* sys, const int32_t* ind_mat, int64_t P_, 
   MQCT_CUDA_TRY(d_W.alloc((size_t)G2 * ldw));
   if (precision == MQCT_PREC_FP64) {
     MQCT_CUDA_TRY(d_acc.alloc((size_t)n_rows * nR));
+    f_shape = contract_fp64_shape(n_tiles, nR, n_sm);
+    const FpShape& fs = kFpShapes[f_shape];
+    MQCT_CUDA_TRY(cudaFuncSetAttribute(fs.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)f_smem(8 * fs.nt * fs.wc)));
   } else {
     int rc2 = tc_init();
     if (rc2) return rc2;
@@ -1167,10 +1252,15 @@ int MatrixPlan::execute(double* d_mat, double* d_y2, int32_t* d_skipped) {
   MQCT_CUDA_TRY(cudaEventRecord(ev[1], stream));
   const FinGrid fg{nR, ir1, ir2, cut, d_spl_fin.p, d_mat, d_skipped, d_y2};
   if (precision == MQCT_PREC_FP64) {
-    dim3 g((n_rows + F_TM - 1) / F_TM, (nR + F_TN - 1) / F_TN);
-    contract_fp64_kernel<<<g, 256, 0, stream>>>(n_rows, G2, nR, d_rowa.p, d_rowb.p, d_psi.p,
-                                                d_W.p, ldw, n_alpha, d_walpha.p, d_acc.p);
-    MQCT_CUDA_TRY(cudaGetLastError());
+    const FpShape& fs = kFpShapes[f_shape];
+    const int tn = 8 * fs.nt * fs.wc;
+    const dim3 g(n_rows / F_TM, (nR + tn - 1) / tn);
+    const int *ra = d_rowa.p, *rb = d_rowb.p;
+    const double2* psi = d_psi.p;
+    const double *W = d_W.p, *wal = d_walpha.p;
+    double* acc = d_acc.p;
+    void* args[] = {&G2, &nR, &ra, &rb, &psi, &W, &ldw, &n_alpha, &wal, &acc};
+    MQCT_CUDA_TRY(cudaLaunchKernel(fs.fn, g, dim3(128 * fs.wc), args, f_smem(tn), stream));
     MQCT_CUDA_TRY(cudaEventRecord(ev[2], stream));
     rc = launch_finalize(fin, P, fg, d_k2r.p, d_acc.p, 1, 0, nR, kCmToHartree, stream);
   } else {

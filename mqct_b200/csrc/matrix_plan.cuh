@@ -102,6 +102,7 @@ struct MatrixPlan {
   DevBuf<double> d_W;     // G2 x ldw, FP64
   int ldw = 0;
   DevBuf<double> d_acc;   // FP64 form: n_rows x nR
+  int f_shape = 0;        // and its tile shape
   DevBuf<double> d_spl_fin;   // grid-only coefficients of the fused spline fit
   DevBuf<double> d_col_scale; // F16x3: exact per-column rescaling of the contraction
 

@@ -99,3 +99,19 @@ def test_build_spline_sizes(mq, gpu_available, nR, prec):
                                 precision=getattr(mq, prec), mij_cutoff=0.0)
     assert np.abs(m).max() > 0 and not sk.any()
     _check_y2(mq, R, m, y2)
+
+
+@pytest.mark.parametrize("jmax,nR,n_alpha", [(2, 31, 0), (2, 33, 3), (6, 33, 0), (6, 48, 0),
+                                             (6, 100, 0), (6, 161, 2), (6, 300, 0), (8, 40, 0),
+                                             (8, 81, 0)])
+def test_build_fp64_tiles(mq, gpu_available, jmax, nR, n_alpha):
+    """The FP64 contraction's tile shapes (chosen by the number of row tiles and R points),
+    ragged columns and grid chunks: an element does not depend on the other radial points, so
+    every third one agrees with a build of those points alone (another shape); 1e-13 of the
+    largest, the two being the same FP64 products and order."""
+    s = mq.CollisionSystem(4, syn.asym_channels(jmax), **dict(A=27.9, B=14.5, C=9.3))
+    R = np.linspace(4.0, 20.0, nR)
+    grid, pes = (9, 7, n_alpha, 0, 0, 0, 1), syn.site_pes(6, seed=4)
+    m, _, _ = mq.build_matrix(s, R, grid, pes, mij_cutoff=0.0)
+    m3, _, _ = mq.build_matrix(s, R[::3], grid, pes, mij_cutoff=0.0)
+    assert np.max(np.abs(m[:, ::3] - m3)) <= 1e-13 * np.abs(m).max()
