@@ -142,8 +142,6 @@ __device__ inline void block_sum3(double& a, double& b, double& c, double* red) 
 }
 
 
-constexpr int kAtCols = 6;  // splined columns of an AT path record
-
 // Cubic-spline value of an AT path column at time t (splint,
 // MQCT_SOURCE_CODES/suppl_routines.f:968-1002).
 __device__ inline double at_splint(const double* rec, const double* y2, int n, int col, int ycol,
@@ -1035,6 +1033,7 @@ struct PropPlan {
   int last_engine = 0;
   LsEngine* ls = nullptr;
   RsEngine* rs = nullptr;
+  OcEngine* oc = nullptr;
   int rs_cl = 0;  // cluster size asked for the resident engine (0: the smallest that fits)
   bool cs = false;  // CS_APPROX for every run of the plan
   int bk_int = 0;                       // bikram_int (ODEINT with per-step stop rules)
@@ -1346,7 +1345,7 @@ struct PropPlan {
       if (rc) return rc;
       float ms = 0.f;
       for (int rep = 0; rep < 2; ++rep) {  // the first launch of a shape loads its code
-        rc = launch(d_probe.p, n, mode, amp.p, cls.p, diag.p);
+        rc = launch_general(d_probe.p, n, mode, amp.p, cls.p, diag.p);
         if (rc) return rc;
         MQCT_CUDA_TRY(cudaEventSynchronize(ev1));
         MQCT_CUDA_TRY(cudaEventElapsedTime(&ms, ev0, ev1));
@@ -1387,11 +1386,30 @@ struct PropPlan {
   // two knot rows and the slot locations.
   double bytes_per_step() const { return 4.0 * (double)S * (4.0 * tsize() + 4.0); }
 
+  // FP64 runs with fixed RK4 steps and no SAVE_TRAJECT records take the one-SM form of the
+  // per-trajectory kernel (onecta.cu) where the tables fit it, whatever the batch: 400 steps of
+  // 48 trajectories (165 states) take 2.5 ms against 8.0, of 600 12.4 against 30.5; tables of 35
+  // states and 2 000 trajectories 6.3 against 43.9; no size that fits was slower.
+  bool use_one_cta(bool records) {
+    if (arith != MQCT_PROP_FP64 || records || method != MQCT_INTEG_RK4 || at_adapt) return false;
+    if (!oc) oc = oc_create();
+    return oc_usable(oc, dev_view(MQCT_MODE_STD), h_blk_n, h_blk_s0, h_blk_slot0, stream);
+  }
+
   int launch(const mqct_traj_init_t* d_init_p, int64_t n_traj, int mode, double* amp,
              double* cls, double* diag, double* rec = nullptr, int64_t rec_cap = 0,
              int64_t* n_rec = nullptr) {
     MQCT_ARG_CHECK(n_traj > 0 && n_traj < (1 << 30), "n_traj out of range");
     last_engine = MQCT_ENGINE_PER_TRAJECTORY;
+    if (use_one_cta(rec != nullptr))
+      return oc_run(oc, dev_view(mode), n_sm, stream, ev0, ev1, d_init_p, (int)n_traj, amp, cls,
+                    diag);
+    return launch_general(d_init_p, n_traj, mode, amp, cls, diag, rec, rec_cap, n_rec);
+  }
+
+  int launch_general(const mqct_traj_init_t* d_init_p, int64_t n_traj, int mode, double* amp,
+                     double* cls, double* diag, double* rec = nullptr, int64_t rec_cap = 0,
+                     int64_t* n_rec = nullptr) {
     MQCT_CUDA_TRY(cudaMemsetAsync(d_queue.p, 0, sizeof(int), stream));
     PropDev d = dev_view(mode);
     TrajOut o{amp, cls, diag, rec, rec_cap, n_rec};
@@ -1554,6 +1572,7 @@ struct PropPlan {
   ~PropPlan() {
     if (ls) ls_destroy(ls);
     if (rs) rs_destroy(rs);
+    if (oc) oc_destroy(oc);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
     if (stream) cudaStreamDestroy(stream);
@@ -1608,7 +1627,8 @@ static int run_host(PropPlan* p, const mqct_traj_init_t* init, int64_t n_traj, i
   for (int64_t t = 0; t < n_traj; ++t) sorted[t] = init[order[t]];
   const bool resident = p->use_resident(mode, n_traj, rec_out != nullptr);
   const bool lockstep = !resident && p->use_lockstep(mode, n_traj, rec_out != nullptr);
-  if (!lockstep && !resident && !p->tuned && p->method == MQCT_INTEG_RK4 && n_traj >= 2LL * p->n_sm) {
+  if (!lockstep && !resident && !p->tuned && p->method == MQCT_INTEG_RK4 &&
+      n_traj >= 2LL * p->n_sm && !p->use_one_cta(rec_out != nullptr)) {
     rc = p->tune(sorted.data(), n_traj, mode);
     if (rc) return rc;
   }

@@ -112,6 +112,22 @@ struct RsResume {
   int counter, status, vib, period, stage, hint, tr;
 };
 
+// Splined columns of an AT path record.
+constexpr int kAtCols = 6;
+
+// The per-trajectory kernel for tables that fit one SM's shared memory (onecta.cu): RK4 in
+// FP64, standard and AT mode, with or without CS.  oc_usable lays it out for the tables (once)
+// and reports whether they fit; oc_run launches it on stream st, ev0 / ev1 bracketing it.
+struct OcEngine;
+OcEngine* oc_create();
+void oc_destroy(OcEngine* e);
+bool oc_usable(OcEngine* e, const PropDev& d, const std::vector<int>& blk_n,
+               const std::vector<int>& blk_s0, const std::vector<int64_t>& blk_slot0,
+               cudaStream_t st);
+int oc_run(OcEngine* e, const PropDev& d, int n_sm, cudaStream_t st, cudaEvent_t ev0,
+           cudaEvent_t ev1, const mqct_traj_init_t* d_init, int n_traj, double* amp, double* cls,
+           double* diag);
+
 // Lockstep engine (lockstep.cu): standard mode, RK4, no CS; every m-block of at most 128
 // states.  ls_run propagates n_traj trajectories whose initial conditions are on the
 // device (d_init) and on the host (h_init, for the bound on the rounds), writing the
