@@ -501,7 +501,7 @@ class MatrixPlan:
         self._sur = sur
 
     def set_drain(self, slices_per_drain):
-        """Alpha points accumulated on the tensor cores between two FP64 drains."""
+        """Alpha points accumulated on the tensor cores between two drains."""
         check(lib().mqct_matrix_plan_set_drain(self.h, int(slices_per_drain)))
 
     def layout(self):

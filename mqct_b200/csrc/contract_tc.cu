@@ -1,33 +1,47 @@
 // contract_tc.cu -- split-precision tensor-core contraction of the matrix build
 // on sm_100a: tcgen05.mma kind::f16 with FP32 accumulators in TMEM, drained into
-// FP64 sums after every short accumulation.
+// sums of two FP32 parts (48 bits) after every short accumulation.
 //
-//   M[row, i] = sum_{c, alpha} w_alpha sum_{g in chunk c} X[row, g] W[g, i]
+//   M[row, i] = w sum_{c, alpha} sum_{g in chunk c} X[row, g] W[g, i]
 //   X = X_hi + X_lo, W = W_hi + W_lo (16-bit parts),
 //   D = X_hi W_hi + X_hi W_lo + X_lo W_hi          (FP32, one K-chunk of 64 points)
-//   S += w_alpha D                                  (FP64, in registers)
+//   S + E += D                                      (S the FP32 sum, E its rounding errors)
 //
 // Two 16-bit formats: BF16x3 (8 significant bits per part, ~16 bits kept) and
 // F16x3 (11 bits per part, ~22 bits kept; the products of FP16 parts are exact
 // in FP32).  FP16's range is narrow, so in F16x3 X is scaled by 2^14 and every
 // radial column of W by the power of two that brings its largest entry to
-// [2^13, 2^14); the exact inverse is applied to the FP64 sums.
+// [2^13, 2^14); the exact inverse is applied to the sums.
 //
 // Accuracy: the tensor core adds the products of one MMA into its FP32
 // accumulator with a rounding relative to the largest addend, so a long
 // accumulation loses bits in proportion to its length and to how much its terms
-// cancel.  Here an accumulator lives for one K-chunk of one alpha point (3 x 4
-// MMAs of K = 16) and is then added to FP64 sums, so every sum over the grid is an
-// FP64 sum of short FP32 partial sums.  The alpha weight multiplies the drained
-// partial in FP64; the tensor-core operand of a K-chunk is the same for every alpha
-// point of a same-m pair (the e^{i m alpha} phases of the two states cancel, so
-// the integrand at every alpha point is w_alpha Re(psi_a^* psi_b) exactly), and the
-// tensor cores contract it once per alpha point.
+// cancel.  Here an accumulator lives for one K-chunk of one group of alpha points (3 x 4 MMAs
+// of K = 16 a point) and is then added to the pair S + E by TwoSum, whose S is exact up to E:
+// against sums in FP64 a build's elements move by 1e-12 (2-norm; the FP32 partials carry 6e-8, the
+// split 5e-6), its error against 64 bits is the same 5.3e-6 (7.0e-6 with an alpha axis).  The
+// ranges of a split axis and the alpha weight (the same for every point of the midpoint grid) are
+// FP64.  The tensor-core operand of a K-chunk is the same for every alpha point of a same-m pair
+// (the e^{i m alpha} phases of the two states cancel, so the integrand at every alpha point is
+// w Re(psi_a^* psi_b) exactly), and the tensor cores contract it once per alpha point.
+//
+// What bounds it, and what the forms before measured (B200; asymmetric top + atom, j <= 8, 31 977
+// pairs, 48 x 48 points, 300 R, whole build; with the 48-point alpha axis):
+//   * FP64 instructions beside MMAs: a drain of converted values into FP64 sums and the MMAs slowed
+//     one another down to half (3 100 clocks a group of two alpha points against 1 750 for its
+//     MMAs alone; the same without the TMEM loads).  In packed FP32 adds: 7.9 -> 5.1 ms;
+//   * the operand X in shared memory was read again by every MMA, 60 clocks of shared-memory
+//     bandwidth for 56 of tensor work.  In TMEM: 5.1 -> 4.9 ms, and 64 KB of shared memory free;
+//   * with one group a chunk (no alpha axis), forming X and the drains alternate in the same
+//     warps: 903 -> 620 us, by the cheaper drain, X through TMEM, accesses that stay in the
+//     shared address space (no spills), and sums stored as whole sectors.
+// The rest is the MMAs (58 to 62 clocks of N = 96 to 112 issued in order by one thread), about 300
+// clocks between two groups, and, without the alpha axis, X.
 //
 // Work unit = one 128-row tile of pair rows (one m-block) x one column part (at
-// most 128 radial points) x one range of K-chunks.  Column parts keep two FP32
-// accumulators of a part in TMEM (double buffering: the tensor cores fill one
-// while the epilogue drains the other) and the FP64 sums of a part in registers.
+// most 112 radial points) x one range of K-chunks.  Two FP32 accumulators of a part in TMEM
+// (double buffering: the tensor cores fill one while the epilogue drains the other) and the
+// sums of a part in registers.
 // Warp roles (64 + 32 PE threads; PE = 16 epilogue warps when a K-chunk has several
 // accumulation groups, 8 when it has one):
 //   warp 0      bulk-copy (TMA) producer: per K-chunk the pre-arranged W image of
@@ -36,13 +50,12 @@
 //               complete_tx, double-buffered where shared memory allows;
 //   warp 1      TMEM allocator + single-thread MMA issuer;
 //   warps 2..   X producers and epilogue: per K-chunk X = Re(psi_a^* psi_b) in FP32
-//               from the staged basis, split to 16-bit hi/lo parts in the
-//               core-matrix layout (PE / 4 threads per tile row); then, for every
-//               alpha point of the chunk, tcgen05.ld of the accumulator and the FP64
-//               update of the sums (PE / 4 warps per TMEM lane quarter, each a share of the
-//               part's columns); at the end of a unit the FP64 sums go to global
-//               memory, one array per K range.
-// The operand tiles use the K-major SWIZZLE_NONE canonical layout: 8 rows x
+//               from the staged basis, split to 16-bit hi/lo parts in TMEM (lane = row, PE / 4
+//               threads per tile row); then, for every group of the chunk, tcgen05.ld of the
+//               accumulator and the update of the sums (PE / 4 warps per TMEM lane quarter, each
+//               a share of the part's columns); at the end of a unit the sums go to global
+//               memory in FP64, one array per K range.
+// W uses the K-major SWIZZLE_NONE canonical layout: 8 rows x
 // 16 B core matrices, K-adjacent core matrices LBO apart, 8-row groups SBO =
 // 128 B apart.  Every mbarrier wait is bounded; on timeout the CTA records an
 // error code, drains, frees its TMEM and returns.
@@ -60,22 +73,22 @@ namespace mqct {
 constexpr int TC_M = 128;        // rows per tile
 constexpr int TC_KC = 64;        // K elements per chunk (8 core-matrix columns of 8 x 16 bit)
 constexpr int TC_PSI_LD = 66;    // float2 per staged basis row (64 + pad)
-// Epilogue warps: a template parameter of the kernel, 8 (two per TMEM lane quarter) or 16
-// (four per lane quarter, for builds with several accumulation groups per K-chunk, where
-// the drain is latency-bound and more warps keep more of it in flight).
+constexpr int TC_NC_MAX = 112;   // columns of one part (TMEM buffer width)
+constexpr int TC_MAX_PARTS = 8;
+constexpr int TC_NLD = 16;       // columns of one TMEM read of the epilogue
+// Tensor memory: two accumulators, then two A stages, each a hi and a lo plane of 16-bit pairs.
+constexpr int TC_A_PLANE = TC_KC / 2;
+constexpr int TC_TMEM_A = 2 * TC_NC_MAX;
+constexpr int TC_TMEM_COLS = 512;  // allocation (a power of two)
+static_assert(TC_TMEM_A + 4 * TC_A_PLANE <= TC_TMEM_COLS, "accumulators and A stages must fit");
+// Epilogue warps: a template parameter of the kernel, 8 (two per TMEM lane quarter) or 16.
 template <int PE>
 struct TcShape {
   static constexpr int THREADS = 64 + 32 * PE;
-  static constexpr int PRODUCERS = 32 * PE;         // X-producer / epilogue threads
-  static constexpr int WPQ = PE / 4;                // epilogue warps per TMEM lane quarter
-  static constexpr int NCH_MAX = PE == 8 ? 56 : 32;  // columns drained by one epilogue thread
+  static constexpr int PRODUCERS = 32 * PE;           // X-producer / epilogue threads
+  static constexpr int WPQ = PE / 4;                  // epilogue warps per TMEM lane quarter
+  static constexpr int NCH_MAX = TC_NC_MAX * 4 / PE;  // columns drained by one epilogue thread
 };
-constexpr int TC_A_PLANE = TC_M * TC_KC * 2;    // bytes of one 16-bit plane of an A stage
-constexpr int TC_NC_MAX = 112;                  // columns of one part (TMEM buffer width)
-constexpr int TC_TMEM_COLS = 256;               // allocation (a power of two >= 2 buffers)
-static_assert(2 * TC_NC_MAX <= TC_TMEM_COLS, "two accumulator buffers must fit the allocation");
-constexpr int TC_MAX_PARTS = 8;
-constexpr int TC_SMEM_ALPHA = 64;                // alpha weights kept in shared memory
 constexpr uint32_t TC_SPIN_LIMIT = kSpinLimit;  // bounded mbarrier waits
 
 // Shared-memory matrix descriptor: K-major, SWIZZLE_NONE, version 1.
@@ -96,12 +109,13 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
 __host__ __device__ constexpr uint32_t idesc_f16(int M, int N) {
   return (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
-__device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc,
+// A from tensor memory (lane = row, two K elements per 32-bit column), B from shared memory.
+__device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint32_t a, uint64_t b, uint32_t idesc,
                                         uint32_t accumulate) {
   asm volatile(
       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
-      "l"(a), "l"(b), "r"(idesc), "r"(accumulate));
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(tmem_d),
+      "r"(a), "l"(b), "r"(idesc), "r"(accumulate));
 }
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
   asm volatile(
@@ -115,22 +129,21 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
 // shared-memory address >> 4 in its low bits), so that the issuing thread does little more
 // than issue: the tensor cores consume a group as fast as one thread issues it.
 template <int Q>
-__device__ __forceinline__ void mma_group(uint32_t td, uint64_t ad0, uint64_t bd0, uint32_t bpl16,
+__device__ __forceinline__ void mma_group(uint32_t td, uint32_t ad0, uint64_t bd0, uint32_t bpl16,
                                           uint32_t bkk16, uint32_t idesc, int nsl) {
-  constexpr uint32_t akk16 = (uint32_t)(2 * (TC_M / 8) * 128) >> 4;
-  constexpr uint32_t apl16 = (uint32_t)TC_A_PLANE >> 4;
   uint32_t acc = 0u;
 #pragma unroll
   for (int pr = 1; pr <= 3; ++pr) {
     const int prod = pr % 3;
     const uint32_t ap = (prod == 2) ? 1u : 0u, bp = (prod == 1) ? 1u : 0u;
-    const uint64_t adp = ad0 + ap * apl16, bdp = bd0 + bp * bpl16;
+    const uint32_t adp = ad0 + ap * TC_A_PLANE;
+    const uint64_t bdp = bd0 + bp * bpl16;
 #pragma unroll
     for (int sl = 0; sl < (Q > 0 ? Q : 1); ++sl) {
       if (Q == 0 && sl >= nsl) break;
 #pragma unroll
       for (int kk = 0; kk < TC_KC / 16; ++kk) {
-        mma_f16(td, adp + kk * akk16, bdp + (uint64_t)(kk * bkk16), idesc, acc);
+        mma_f16(td, adp + kk * 8, bdp + (uint64_t)(kk * bkk16), idesc, acc);
         acc = 1u;
       }
     }
@@ -138,21 +151,74 @@ __device__ __forceinline__ void mma_group(uint32_t td, uint64_t ad0, uint64_t bd
       for (int sl = 1; sl < nsl; ++sl)
 #pragma unroll
         for (int kk = 0; kk < TC_KC / 16; ++kk)
-          mma_f16(td, adp + kk * akk16, bdp + (uint64_t)(kk * bkk16), idesc, 1u);
+          mma_f16(td, adp + kk * 8, bdp + (uint64_t)(kk * bkk16), idesc, 1u);
     }
   }
 }
 // 8 consecutive TMEM columns of this warp's lane quarter (one 32-bit value per lane each);
 // the values are valid after tmem_wait().
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,"
+      "%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+        "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t* r) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
         "=r"(r[7])
       : "r"(taddr));
 }
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t* r) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_st4(uint32_t taddr, const uint4& v) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(taddr), "r"(v.x),
+               "r"(v.y), "r"(v.z), "r"(v.w)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() {
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
 __device__ __forceinline__ void tmem_wait() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+// (no use of x moves ahead of a wait before it)
+__device__ __forceinline__ void tmem_landed(uint32_t& x) { asm volatile("" : "+r"(x)); }
+
+// Two columns' sums as FP32 pairs, value S + E: TwoSum (Knuth) of S and the drained value x,
+// with the rounding error of S, which it gives exactly, added to E.
+struct F32x2 {
+  unsigned long long v;
+};
+__device__ __forceinline__ F32x2 add2(F32x2 a, F32x2 b) {
+  F32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F32x2 sub2(F32x2 a, F32x2 b) {
+  F32x2 r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F32x2 pack2(uint32_t a, uint32_t b) {
+  return F32x2{(unsigned long long)b << 32 | a};
+}
+__device__ __forceinline__ void two_sum(F32x2& S, F32x2& E, F32x2 x) {
+  const F32x2 t = add2(S, x), z = sub2(t, S);
+  E = add2(E, add2(sub2(S, sub2(t, z)), sub2(x, z)));
+  S = t;
+}
+// S + E in FP64; an infinite or NaN sum stays what it is.
+__device__ __forceinline__ double pair_value(uint32_t s, uint32_t e) {
+  const float f = __uint_as_float(s);
+  return isfinite(f) ? (double)f + (double)__uint_as_float(e) : (double)f;
 }
 
 __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
@@ -342,20 +408,20 @@ __device__ __forceinline__ uint32_t empty_parity(uint32_t k, uint32_t nb) {
   return ((k / nb) + 1u) & 1u;
 }
 
-template <bool kF16, int PE>
+// kMulti: several accumulation groups a chunk are possible (its code costs the eight-warp form
+// registers: 613 -> 650 us of the j <= 8 build).
+template <bool kF16, int PE, bool kMulti>
 __global__ void __launch_bounds__(TcShape<PE>::THREADS, 1) tc_contract_kernel(TcArgs a) {
   constexpr int TC_THREADS = TcShape<PE>::THREADS, TC_PRODUCERS = TcShape<PE>::PRODUCERS;
   constexpr int TC_KSPLIT = TC_PRODUCERS / TC_M;  // threads per tile row in X production
   constexpr int TC_WPQ = TcShape<PE>::WPQ, TC_NCH_MAX = TcShape<PE>::NCH_MAX;
   static_assert(TC_PRODUCERS % TC_M == 0 && (TC_KC / 8) % TC_KSPLIT == 0, "X production split");
-  static_assert((TC_NC_MAX / 8 + TC_WPQ - 1) / TC_WPQ <= TC_NCH_MAX / 8, "drain split");
+  static_assert(TC_NC_MAX <= TC_WPQ * TC_NCH_MAX && 16 % TC_WPQ == 0, "drain split");
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  uintptr_t base = (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023);
-  unsigned char* sB = reinterpret_cast<unsigned char*>(base);           // nbuf x b_stage
+  // (an offset, not a rounded integer: the accesses stay in the shared address space)
+  unsigned char* sB = smem_raw + ((0u - smem_u32(smem_raw)) & 1023u);    // nbuf x b_stage
   unsigned char* sPsi = sB + a.nbuf * a.b_stage;                         // nbuf x psi_stage
-  unsigned char* sA = sPsi + a.nbuf * a.psi_stage;                       // 2 x A stage
-  const uint32_t a_stage = 2u * TC_A_PLANE;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sA + 2 * a_stage);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sPsi + a.nbuf * a.psi_stage);
   uint64_t* B_full = bars;          // [2]
   uint64_t* B_empty = bars + 2;     // [2]
   uint64_t* P_full = bars + 4;      // [2]
@@ -368,22 +434,17 @@ __global__ void __launch_bounds__(TcShape<PE>::THREADS, 1) tc_contract_kernel(Tc
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 19);
 
-  // the alpha weights in shared memory: the epilogue reads one per drain, and a global
-  // load there would sit on the drain's critical path
-  __shared__ double s_walpha[TC_SMEM_ALPHA];
-  for (int i = threadIdx.x; i < TC_SMEM_ALPHA; i += TC_THREADS)
-    s_walpha[i] = (a.walpha && i < a.n_alpha_it) ? a.walpha[i] : 1.0;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < 2; ++s) {
       mbar_init(&B_full[s], 1);
       mbar_init(&B_empty[s], 1);
       mbar_init(&P_full[s], 1);
-      mbar_init(&P_empty[s], TC_PRODUCERS);
-      mbar_init(&A_full[s], TC_PRODUCERS);
+      mbar_init(&P_empty[s], PE);  // one arrival per warp: 512 on one barrier took 1 000 clocks
+      mbar_init(&A_full[s], PE);
       mbar_init(&A_empty[s], 1);
       mbar_init(&ACC_full[s], 1);
-      mbar_init(&ACC_empty[s], TC_PRODUCERS);
+      mbar_init(&ACC_empty[s], PE);
     }
     mbar_init(DONE, 1);
     *abort_flag = 0;
@@ -439,8 +500,7 @@ __global__ void __launch_bounds__(TcShape<PE>::THREADS, 1) tc_contract_kernel(Tc
     // ---------------- MMA issuer
     if (lane == 0) {
       uint32_t kc = 0, ka = 0, kacc = 0;  // chunk uses, A-stage uses, accumulator uses
-      const uint32_t sA0 = smem_u32(sA), sB0 = smem_u32(sB);
-      const uint32_t lbo_a = (TC_M / 8) * 128;
+      const uint32_t sB0 = smem_u32(sB);
       for (int u = blockIdx.x; u < a.n_units && !*abort_flag; u += gridDim.x) {
         const int ks = u % a.n_ks, pt = (u / a.n_ks) % a.n_parts;
         const int nc = a.parts.nc[pt];
@@ -454,9 +514,9 @@ __global__ void __launch_bounds__(TcShape<PE>::THREADS, 1) tc_contract_kernel(Tc
                mbar_wait(&A_full[sa], full_parity(ka, 2), abort_flag, a.status, 22);
           if (!ok) break;
           tc_fence_after();
-          const uint32_t aoff = sA0 + sa * (2 * TC_A_PLANE);
+          const uint32_t ad0 = tmem + TC_TMEM_A + sa * (2 * TC_A_PLANE);
           const uint32_t boff0 = sB0 + sb * a.b_stage;
-          const uint64_t ad0 = smem_desc(aoff, lbo_a, 128), bd0 = smem_desc(boff0, lbo_b, 128);
+          const uint64_t bd0 = smem_desc(boff0, lbo_b, 128);
           const uint32_t bpl16 = bplane >> 4, bkk16 = (2 * lbo_b) >> 4;
           for (int al = 0; al < a.n_alpha_it; ++al, ++kacc) {
             const uint32_t sc = kacc & 1u;
@@ -489,25 +549,22 @@ __global__ void __launch_bounds__(TcShape<PE>::THREADS, 1) tc_contract_kernel(Tc
     }
   } else {
     // ---------------- X producers (warps 2 to PE + 1) and epilogue
-    const int t = threadIdx.x - 64;
-    const int p = t & (TC_M - 1);  // tile row generated by this thread
-    const int kh = t / TC_M;       // share of the chunk's K groups formed by this thread
     const int q = warp & 3;        // TMEM lane quarter accessible to this warp
-    const int h = (warp - 2) >> 2; // share of the part's columns drained by this warp
+    const int h = (warp - 2) >> 2; // its share of a chunk's K groups and of a part's columns
+    const int p = q * 32 + lane;   // the thread's tile row
     uint32_t kc = 0, ka = 0, kacc = 0;
-    double S[TC_NCH_MAX];
+    const double wa = a.walpha ? a.walpha[0] : 1.0;  // every alpha point's weight
+    F32x2 S[TC_NCH_MAX / 2], E[TC_NCH_MAX / 2];
     for (int u = blockIdx.x; u < a.n_units && !*abort_flag; u += gridDim.x) {
       const int ks = u % a.n_ks, pt = (u / a.n_ks) % a.n_parts, tile = u / (a.n_ks * a.n_parts);
       const int blk = a.tile_block[tile];
       const int row = tile * TC_M + p;
       const int la = a.rowa[row] - a.blk_row0[blk], lb = a.rowb[row] - a.blk_row0[blk];
-      // the part's batches of 8 columns split over the warps of a lane quarter
-      const int nb8 = a.parts.nc[pt] / 8;
-      const int b8lo = h * nb8 / TC_WPQ, b8hi = (h + 1) * nb8 / TC_WPQ;
-      const int nch = 8 * (b8hi - b8lo), coff = 8 * b8lo, col0 = a.parts.c0[pt] + coff;
+      // the part's columns (a multiple of 16) split over the warps of a lane quarter
+      const int nch = a.parts.nc[pt] / TC_WPQ, coff = h * nch, col0 = a.parts.c0[pt] + coff;
       const int c0 = ks * a.chunks_per_ks, c1 = min(a.n_chunks, c0 + a.chunks_per_ks);
 #pragma unroll
-      for (int i = 0; i < TC_NCH_MAX; ++i) S[i] = 0.0;
+      for (int i = 0; i < TC_NCH_MAX / 2; ++i) S[i].v = E[i].v = 0;
       // produce the operand of chunk use kcu into A stage (kau & 1) from basis slice
       // (kcu % nbuf)
       auto produce = [&](uint32_t kcu, uint32_t kau) -> bool {
@@ -515,14 +572,15 @@ __global__ void __launch_bounds__(TcShape<PE>::THREADS, 1) tc_contract_kernel(Tc
         if (!mbar_wait(&P_full[sp], full_parity(kcu, nbuf), abort_flag, a.status, 31)) return false;
         if (kau >= 2 && !mbar_wait(&A_empty[sa], empty_parity(kau, 2), abort_flag, a.status, 32))
           return false;
+        tc_fence_after();
+        __syncwarp();
         const float2* ps = reinterpret_cast<const float2*>(sPsi + sp * a.psi_stage);
         const float2* pa = ps + la * TC_PSI_LD;
         const float2* pb = ps + lb * TC_PSI_LD;
-        unsigned char* hi = sA + sa * (2 * TC_A_PLANE);
-        unsigned char* lo = hi + TC_A_PLANE;
+        const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + TC_TMEM_A + sa * (2 * TC_A_PLANE);
 #pragma unroll
         for (int kq = 0; kq < TC_KC / 8 / TC_KSPLIT; ++kq) {
-          const int kg = kh * (TC_KC / 8 / TC_KSPLIT) + kq;
+          const int kg = h * (TC_KC / 8 / TC_KSPLIT) + kq;
           float x[8];
 #pragma unroll
           for (int e = 0; e < 8; e += 2) {
@@ -537,13 +595,16 @@ __global__ void __launch_bounds__(TcShape<PE>::THREADS, 1) tc_contract_kernel(Tc
           }
           uint4 hv, lv;
           split8<kF16>(x, hv, lv);
-          const uint32_t off = (uint32_t)(kg * (TC_M / 8) + (p >> 3)) * 128u + (uint32_t)(p & 7) * 16u;
-          *reinterpret_cast<uint4*>(hi + off) = hv;
-          *reinterpret_cast<uint4*>(lo + off) = lv;
+          tmem_st4(ta + kg * 4, hv);
+          tmem_st4(ta + TC_A_PLANE + kg * 4, lv);
         }
-        fence_proxy_async();
-        mbar_arrive(&A_full[sa]);
-        mbar_arrive(&P_empty[sp]);
+        tmem_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+          mbar_arrive(&A_full[sa]);
+          mbar_arrive(&P_empty[sp]);
+        }
         return true;
       };
       // With two B / basis buffers the next chunk's operand is formed before this chunk
@@ -563,39 +624,66 @@ __global__ void __launch_bounds__(TcShape<PE>::THREADS, 1) tc_contract_kernel(Tc
             break;
           }
           tc_fence_after();
-          // a group of several alpha points shares one (uniform) weight
-          const double wa = al < TC_SMEM_ALPHA ? s_walpha[al] : (a.walpha ? a.walpha[al] : 1.0);
+          __syncwarp();
           const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + sc * TC_NC_MAX + (uint32_t)coff;
-          // batches of 8 columns, software-pipelined: the next batch's TMEM load is in
-          // flight while this batch is added to the FP64 sums
-          constexpr int NB8 = TC_NCH_MAX / 8;
-          uint32_t r[2][8];
-          tmem_ld8(taddr, r[0]);
-          tmem_wait();
+          // batches of columns; after the last load the accumulator is free
 #pragma unroll
-          for (int b8 = 0; b8 < NB8; ++b8) {
-            if (8 * b8 < nch) {  // the same for the whole warp
-              const bool more = 8 * (b8 + 1) < nch;
-              if (more) tmem_ld8(taddr + 8 * (b8 + 1), r[(b8 + 1) & 1]);
-#pragma unroll
-              for (int e = 0; e < 8; ++e) {
-                double& acc = S[8 * b8 + e];
-                acc = fma((double)__uint_as_float(r[b8 & 1][e]), wa, acc);
+          for (int b0 = 0; b0 < TC_NCH_MAX; b0 += TC_NLD) {  // conditions alike for the warp
+            uint32_t r[TC_NLD];
+            const int m = nch - b0;
+            if (m > 0) {
+              if (b0 + 16 <= TC_NCH_MAX && m >= 16) {
+                tmem_ld16(taddr + b0, r);
+              } else {
+                if (m >= 8) tmem_ld8(taddr + b0, r);
+                if (m >= 12) tmem_ld4(taddr + b0 + 8, r + 8);
+                else if (m == 4) tmem_ld4(taddr + b0, r);
               }
-              if (more) tmem_wait();
+              tmem_wait();
+            }
+            if (b0 + TC_NLD >= TC_NCH_MAX) {
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(&ACC_empty[sc]);
+            }
+#pragma unroll
+            for (int i = 0; i < TC_NLD && b0 + i < TC_NCH_MAX; i += 4) {
+              if (i >= m) break;
+#pragma unroll
+              for (int e = i; e < i + 4; ++e) tmem_landed(r[e]);
+              two_sum(S[(b0 + i) / 2], E[(b0 + i) / 2], pack2(r[i], r[i + 1]));
+              two_sum(S[(b0 + i) / 2 + 1], E[(b0 + i) / 2 + 1], pack2(r[i + 2], r[i + 3]));
             }
           }
-          tc_fence_before();
-          mbar_arrive(&ACC_empty[sc]);
+        }
+        if (kMulti && a.n_alpha_it > a.slices_per_drain) {  // E stays below an ulp of S
+#pragma unroll
+          for (int i = 0; i < TC_NCH_MAX / 2; ++i) {
+            const F32x2 t = add2(S[i], E[i]);
+            E[i] = sub2(E[i], sub2(t, S[i]));
+            S[i] = t;
+          }
         }
         if (ok && !ahead && c + 1 < c1 && !produce(kc + 1, ka + 1)) ok = false;
       }
       if (!ok) break;
-      // the unit's FP64 sums, with the exact column factors
-      double* dst = a.part + (int64_t)ks * a.part_stride + (int64_t)(tile * TC_M + q * 32 + lane) * a.ldp;
+      // the unit's sums in FP64, with the alpha weight and the exact column factors
+      double* dst = a.part + (int64_t)ks * a.part_stride + (int64_t)row * a.ldp;
 #pragma unroll
-      for (int i = 0; i < TC_NCH_MAX; ++i)
-        if (i < nch) dst[col0 + i] = S[i] * a.col_scale[col0 + i];
+      for (int i = 0; i < TC_NCH_MAX; i += 4)
+        if (i < nch) {
+          double v[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int h32 = 32 * (e & 1), j = (i + e) / 2;
+            v[e] = wa * pair_value((uint32_t)(S[j].v >> h32), (uint32_t)(E[j].v >> h32)) *
+                   __ldg(a.col_scale + col0 + i + e);
+          }
+          // whole 32-byte sectors: 16-byte stores took 11 000 clocks of a 128 x 112 unit
+          asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(dst + col0 + i), "d"(v[0]),
+                       "d"(v[1]), "d"(v[2]), "d"(v[3])
+                       : "memory");
+        }
     }
   }
   tc_fence_before();
@@ -608,6 +696,16 @@ __global__ void __launch_bounds__(TcShape<PE>::THREADS, 1) tc_contract_kernel(Tc
 }
 
 // ---------------------------------------------------------------- host side
+static const void* tc_kernel(bool f16, bool many, bool multi) {
+  if (many)
+    return f16 ? (const void*)tc_contract_kernel<true, 16, true>
+               : (const void*)tc_contract_kernel<false, 16, true>;
+  if (multi)
+    return f16 ? (const void*)tc_contract_kernel<true, 8, true>
+               : (const void*)tc_contract_kernel<false, 8, true>;
+  return f16 ? (const void*)tc_contract_kernel<true, 8, false>
+             : (const void*)tc_contract_kernel<false, 8, false>;
+}
 int MatrixPlan::tc_init() {
   MQCT_ARG_CHECK(nR <= TC_NC_MAX * TC_MAX_PARTS, "tensor-core contraction supports nR <= %d (got %d)",
                  TC_NC_MAX * TC_MAX_PARTS, nR);
@@ -650,14 +748,8 @@ int MatrixPlan::tc_init() {
   t.psi_stage = (uint32_t)up((size_t)t.nbmax * TC_PSI_LD * 8);
   int dev_smem = 0;
   cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  {
-    // the kernel's static shared memory (the alpha weights) comes out of the same budget
-    cudaFuncAttributes fa{};
-    MQCT_CUDA_TRY(cudaFuncGetAttributes(&fa, tc_contract_kernel<true, 16>));
-    dev_smem -= (int)fa.sharedSizeBytes;
-  }
   for (t.nbuf = 2; t.nbuf >= 1; --t.nbuf) {
-    t.smem = 1024 + (size_t)t.nbuf * (t.b_stage + t.psi_stage) + 2ull * 2 * TC_A_PLANE + 256;
+    t.smem = 1024 + (size_t)t.nbuf * (t.b_stage + t.psi_stage) + 256;
     if (t.smem <= (size_t)dev_smem) break;
   }
   MQCT_ARG_CHECK(t.nbuf >= 1, "shared memory too small for the tcgen05 tiles (nR=%d, block %d)",
@@ -669,23 +761,30 @@ int MatrixPlan::tc_init() {
   MQCT_CUDA_TRY(t.blk_m.upload(bm, stream));
   MQCT_CUDA_TRY(t.blk_img_off.upload(off, stream));
   if (n_alpha > 0) MQCT_CUDA_TRY(t.walpha.upload(h_walpha, stream));
-  // alpha points per drain: a group shares one weight, so groups of more than one point
-  // need equal weights (the midpoint alpha grid); 2 keeps the drains under the MMA time
+  // alpha points per drain: 2 keeps the drains under the MMA time.  The weight is applied to the
+  // sums: it is the same for every point of the midpoint grid, the only alpha grid there is.
   t.alpha_uniform = true;
   for (int i = 1; i < n_alpha; ++i)
     if (h_walpha[i] != h_walpha[0]) t.alpha_uniform = false;
+  MQCT_ARG_CHECK(t.alpha_uniform, "the tcgen05 contraction needs equal alpha weights");
   t.slices_per_drain = (n_alpha > 1 && t.alpha_uniform) ? 2 : 1;
-  // K ranges: split the chunks only to fill the last wave of units (the FP64 sums of
-  // every range are written once and added by the finalize)
+  // K ranges: split the chunks only to fill the last wave of units, or the SMs when the units of
+  // one range are fewer (the FP64 sums of every range are written once and added by the
+  // finalize).  The cost of ks ranges, in accumulation groups: a chunk's groups and its X, and 15
+  // for a unit's start, its sums and their way through the finalize (asymmetric top, j <= 8,
+  // 771 units a range: 636, 649, 690 and 766 us for 1 to 4 ranges; with 24 groups a chunk 5 394,
+  // 5 077, 4 922 and 5 120; two tops, 13 units: 5 555, 4 027, 3 662 and 3 497 for 1, 4, 8, 11).
   cudaDeviceGetAttribute(&t.n_sm, cudaDevAttrMultiProcessorCount, dev);
+  const int64_t units1 = (int64_t)n_tiles * t.n_parts;
+  const int ks_max = std::min(units1 < t.n_sm ? 16 : 4, t.n_chunks);
+  const int groups = (std::max(1, n_alpha) + t.slices_per_drain - 1) / t.slices_per_drain;
   int best_ks = 1;
-  double best_eff = 0.0;
-  for (int ks = 1; ks <= std::min(4, t.n_chunks); ++ks) {
-    const double units = (double)n_tiles * t.n_parts * ks;
-    const double waves = units / t.n_sm;
-    const double eff = waves / std::ceil(waves) - 0.01 * (ks - 1);  // partial-sum traffic
-    if (eff > best_eff + 1e-9) {
-      best_eff = eff;
+  double best = 0.0;
+  for (int ks = 1; ks <= ks_max; ++ks) {
+    const int cps = (t.n_chunks + ks - 1) / ks, ns = (t.n_chunks + cps - 1) / cps;
+    const double cost = (double)((units1 * ns + t.n_sm - 1) / t.n_sm) * (cps * (groups + 1) + 15);
+    if (ks == 1 || cost < best) {
+      best = cost;
       best_ks = ks;
     }
   }
@@ -715,18 +814,13 @@ int MatrixPlan::tc_init() {
   if (precision == MQCT_PREC_F16X3) {
     MQCT_CUDA_TRY(t.wmax.alloc((size_t)nR));
     MQCT_CUDA_TRY(cudaMemsetAsync(d_col_scale.p, 0, sizeof(double) * t.npad, stream));
-    MQCT_CUDA_TRY(cudaFuncSetAttribute(tc_contract_kernel<true, 8>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)t.smem));
-    MQCT_CUDA_TRY(cudaFuncSetAttribute(tc_contract_kernel<true, 16>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)t.smem));
   } else {
     std::vector<double> ones(t.npad, 1.0);
     MQCT_CUDA_TRY(d_col_scale.upload(ones, stream));
-    MQCT_CUDA_TRY(cudaFuncSetAttribute(tc_contract_kernel<false, 8>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)t.smem));
-    MQCT_CUDA_TRY(cudaFuncSetAttribute(tc_contract_kernel<false, 16>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)t.smem));
   }
+  for (int f = 0; f < 3; ++f)
+    MQCT_CUDA_TRY(cudaFuncSetAttribute(tc_kernel(precision == MQCT_PREC_F16X3, f == 2, f == 1),
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)t.smem));
   return MQCT_OK;
 }
 
@@ -797,13 +891,11 @@ int MatrixPlan::tc_execute() {
   const bool many = t.pe_force ? t.pe_force == 16
                                : (a.n_alpha_it + a.slices_per_drain - 1) / a.slices_per_drain >= 2;
   t.pe_warps = many ? 16 : 8;
-  if (f16) {
-    if (many) tc_contract_kernel<true, 16><<<grid, TcShape<16>::THREADS, t.smem, stream>>>(a);
-    else tc_contract_kernel<true, 8><<<grid, TcShape<8>::THREADS, t.smem, stream>>>(a);
-  } else {
-    if (many) tc_contract_kernel<false, 16><<<grid, TcShape<16>::THREADS, t.smem, stream>>>(a);
-    else tc_contract_kernel<false, 8><<<grid, TcShape<8>::THREADS, t.smem, stream>>>(a);
-  }
+  const bool multi = a.n_alpha_it > a.slices_per_drain;
+  void* args[] = {&a};
+  MQCT_CUDA_TRY(cudaLaunchKernel(tc_kernel(f16, many, multi), dim3(grid),
+                                 dim3(many ? TcShape<16>::THREADS : TcShape<8>::THREADS), args,
+                                 t.smem, stream));
   MQCT_CUDA_TRY(cudaGetLastError());
   return MQCT_OK;
 }

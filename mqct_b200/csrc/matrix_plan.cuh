@@ -25,7 +25,7 @@ struct TcInfo {
   int n_chunks = 0, chunks_per_split = 1, npad = 0, nbmax = 0;
   int n_parts = 1, part_c0[8] = {}, part_nc[8] = {};  // column parts of the radial axis
   int nbuf = 2;                                        // B / basis-slice buffers
-  int slices_per_drain = 1;                            // alpha points per FP64 drain
+  int slices_per_drain = 1;                            // alpha points per drain
   bool alpha_uniform = true;                           // all alpha weights equal
   int pe_warps = 8;                                    // epilogue warps of the last launch
   int pe_force = 0;                                    // 8 or 16 (tuned or set), 0: by rule
