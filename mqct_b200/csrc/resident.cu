@@ -529,7 +529,7 @@ __global__ void __launch_bounds__(RS_THREADS, 1) rs_kernel(PropDev d, RsDev D) {
           amp[d.N + w.ri] = 0.0;
         }
       }
-      if (go) rs_phases(PH[rc & 1], ev, D.n_e, 0.0);
+      if (go) rs_phases(PH[rc & 1], ev, D.n_e, S.tcur);
     }
     clu.sync();  // the peers read these amplitudes from the first right-hand side on
     if (!go) continue;
