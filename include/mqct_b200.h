@@ -230,7 +230,7 @@ double mqct_matrix_plan_flops(const mqct_matrix_plan* plan);
  * are added to sums of two FP32 parts (48 bits) after every group of slices_per_drain alpha
  * points of a 64-point grid chunk (1..64; more than 1 needs equal alpha weights; the plan's choice is
  * 2 on an equal-weight alpha grid, else 1).  mqct_matrix_plan_layout reports that choice,
- * the number of grid-chunk ranges whose FP64 sums the finalize adds, and the number of
+ * the number of grid-chunk ranges whose sums the finalize adds in FP64, and the number of
  * radial column parts (0 for the FP64 form). */
 int mqct_matrix_plan_set_drain(mqct_matrix_plan* plan, int32_t slices_per_drain);
 int mqct_matrix_plan_layout(const mqct_matrix_plan* plan, int32_t* slices_per_drain,

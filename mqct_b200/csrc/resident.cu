@@ -15,22 +15,30 @@
 // loaded again only when the stage point leaves the interval (one of the two rows is
 // kept when the neighbour interval is entered).
 //
-// Per right-hand side every CTA of the cluster
-//   * forms the stage point's scalars and spline factors (thread 0; the same values in
-//     every CTA, from the same classical state),
-//   * bt = D^* a and u = (J_+ + J_-) a for its rows, the neighbour amplitudes of u read
-//     from the owning CTA's shared memory when another CTA holds them (distributed
-//     shared memory),
-//   * interpolates its blocks' matrix elements into a packed triangle (M) and adds its
-//     part of the force Re(bt^+ M' bt), then y = M bt for its rows,
-//   * forms da = -i e^{iEt} y - i (dphi/2) u and the RK4 update of its rows, and its parts
-//     of F, g = Im((D^* u)^+ y) and pot = Re(bt^+ y),
-//   * writes its three parts into every CTA of the cluster and waits at the cluster
-//     barrier (one per right-hand side),
-// after which each CTA adds the CL parts in rank order and takes the classical RK4 stage
-// itself: every CTA holds the same classical state, bit for bit, so the stop decisions
-// agree without another exchange.  CTA rank 0 takes the next trajectory from a device
-// queue and hands its index to the others.
+// R of a point depends on the momentum of the point before it, not on its force, so the
+// spline interval and factors of a right-hand side are known one right-hand side ahead, and
+// nothing before its rows' derivatives waits for the sums of the one before.  Per right-hand
+// side every CTA of the cluster
+//   * forms bt = D^* a for its rows and interpolates its blocks' matrix elements into a packed
+//     triangle (M), adding its part of the force Re(bt^+ M' bt), while a warp of its own, the
+//     classical warp, adds the cluster's parts of the right-hand side before, takes its
+//     classical RK4 stage (dphi/dt of this point, the stop rules) and prepares the next point;
+//   * forms y = M bt, u = (J_+ + J_-) a, da = -i e^{iEt} y - i (dphi/2) u and the RK4 update of
+//     its rows, and its parts of F, g = Im((D^* u)^+ y) and pot = Re(bt^+ y); a row's new stage
+//     input is pushed into the shared memory of the CTAs that hold its Coriolis neighbours;
+//   * every warp writes its three parts into every CTA of the cluster, and the CTAs meet at the
+//     cluster barrier (one per right-hand side); two warps form the next phases beside the rows.
+// Every CTA adds the parts in the same order and holds the same classical state, bit for bit,
+// so the stop decisions agree without another exchange.  CTA rank 0 takes the next trajectory
+// from a device queue and hands its index to the others.
+//
+// What bounds it: shared-memory wavefronts and instruction issue of the slots and the rows, one
+// after the other (about 6 us of an evaluation by four CTAs).  Before, one thread summed the
+// parts, took the classical stage and prepared the point between the cluster barrier and the
+// next evaluation, with four block barriers in each: 48 trajectories on the 969-state tables
+// (300 R, 700-2000 cm^-1) took 185 ms, now 170 (clusters of four; the same bits).  Keeping a
+// thread's slot indices and some of its knots in registers spills under the 96 registers that
+// eighteen warps leave: 199 ms.
 //
 // The arithmetic of a right-hand side is that of the per-trajectory kernel in FP32 (the
 // slots interpolated one by one, the same products); sums run over other partitions, so
@@ -48,7 +56,8 @@ namespace cg = cooperative_groups;
 namespace mqct {
 
 constexpr int RS_THREADS = 512;
-constexpr int RS_WARPS = RS_THREADS / 32;
+constexpr int RS_WARPS = RS_THREADS / 32;  // row warps; the classical warp and one more follow
+constexpr int RS_BLOCK = RS_THREADS + 64;
 constexpr int RS_MAX_CL = 8;
 constexpr int RS_MAX_BLK = 64;   // blocks per CTA
 constexpr int RS_MAX_STATES = 255;  // states of one m-block (8-bit local row indices)
@@ -57,17 +66,21 @@ constexpr int RS_MAX_STATES = 255;  // states of one m-block (8-bit local row in
 struct RsCls {
   Cls C, CT, K1, K23;                 // state, stage point, first-stage and middle-stage sums
   double tcur, dt, eki, eqi, tmpR1, tmpR2;
-  double th_c, sin_c, is2_c;          // theta of the cached sine and 1/sin^2
-  double dphidt, sin_t, inv_r, inv_s2;
-  float cf[7];                        // M: aa, bb, c1, c2;  M': 1/h, d1, d2
+  double sin_t, inv_s2;               // of theta, which no stage changes
   int counter, status, vib, period;
   int stage;                          // 0..3 RK4 stages, 4 closing evaluation, 5 done
-  int key;                            // spline interval of the stage point; nR - 1 above
   int hint;
   int s_int;
+  int tag[2];                         // knot row held by buffer 0 / 1, or -1
+};
+
+// The point of a right-hand side: formed one right-hand side ahead, but for dphidt.
+struct RsPoint {
+  double R, inv_r, dphidt;
+  float cf[7];                        // M: aa, bb, c1, c2;  M': 1/h, d1, d2
+  int key;                            // spline interval; nR - 1 above the grid
   int lo_buf;                         // knot buffer holding row key (the other: key + 1)
   int load[2];                        // knot row to load into buffer 0 / 1, or -1
-  int tag[2];                         // knot row held by buffer 0 / 1, or -1
 };
 
 // One row (state) of a CTA: what its right-hand-side terms need, fixed for the tables.
@@ -104,10 +117,10 @@ struct RsDev {
 
 // Dynamic shared memory of one CTA (offsets in bytes, 16-byte aligned).
 struct RsSmem {
-  size_t kn0, kn1, mp, loc, y64, acc, ain0, ain1, halo0, halo1, bt, u, ph0, ph1, rows, rg, ih,
-      ev, total;
+  size_t kn0, kn1, mp, loc, y64, acc, ain0, ain1, halo0, halo1, bt, ph0, ph1, rows, rg, ih,
+      ev, part, total;
 };
-__host__ __device__ inline RsSmem rs_layout(int ns_cap, int nr_cap, int n_e, int nR) {
+__host__ __device__ inline RsSmem rs_layout(int ns_cap, int nr_cap, int n_e, int nR, int CL) {
   RsSmem s{};
   size_t o = 0;
   auto take = [&](size_t bytes) {
@@ -126,35 +139,47 @@ __host__ __device__ inline RsSmem rs_layout(int ns_cap, int nr_cap, int n_e, int
   s.halo0 = take((size_t)nr_cap * 16);
   s.halo1 = take((size_t)nr_cap * 16);
   s.bt = take((size_t)nr_cap * 8);
-  s.u = take((size_t)nr_cap * 8);
   s.ph0 = take((size_t)n_e * 8);
   s.ph1 = take((size_t)n_e * 8);
   s.rows = take((size_t)nr_cap * sizeof(RsRow));
   s.rg = take((size_t)nR * 8);
   s.ih = take((size_t)nR * 8);
   s.ev = take((size_t)n_e * 8);
+  s.part = take((size_t)2 * CL * RS_WARPS * 3 * 8);
   s.total = o;
   return s;
 }
 
-// Warp sums of three doubles (fixed tree) into red[3 w + q]; the block's barrier follows.
-__device__ inline void rs_warp_parts(double a, double b, double c, double* red) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+// Warp sums of three doubles (fixed tree), in every lane.
+__device__ inline void rs_warp_sum3(double& a, double& b, double& c) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     a += __shfl_xor_sync(0xffffffffu, a, o);
     b += __shfl_xor_sync(0xffffffffu, b, o);
     c += __shfl_xor_sync(0xffffffffu, c, o);
   }
-  if (lane == 0) {
-    red[3 * w] = a;
-    red[3 * w + 1] = b;
-    red[3 * w + 2] = c;
-  }
-  __syncthreads();
 }
 
-// Start of a trajectory (thread 0): MQCT_SOURCE_CODES/propagator.f:2531-2566.  Returns
+// The cluster's sums from the parts of its warps, [CL][RS_WARPS][3] (one warp; the sums in every
+// lane): per CTA and quantity the warps in order, then the CTAs in order.
+__device__ inline void rs_sums(const double* part, int CL, double& a, double& b, double& c) {
+  const int lane = threadIdx.x & 31;
+  static_assert(3 * RS_MAX_CL <= 32, "a lane per CTA and quantity");
+  double v = 0.0;
+  if (lane < 3 * CL) {
+    const double* p = part + (lane / 3) * RS_WARPS * 3 + lane % 3;
+#pragma unroll
+    for (int i = 0; i < RS_WARPS; ++i) v += p[3 * i];
+  }
+  a = b = c = 0.0;
+  for (int r = 0; r < CL; ++r) {
+    a += __shfl_sync(0xffffffffu, v, 3 * r);
+    b += __shfl_sync(0xffffffffu, v, 3 * r + 1);
+    c += __shfl_sync(0xffffffffu, v, 3 * r + 2);
+  }
+}
+
+// Start of a trajectory (one thread): MQCT_SOURCE_CODES/propagator.f:2531-2566.  Returns
 // false for a trajectory that is not propagated (l / k above R_start, status 2), whose
 // classical and diagnostic outputs rank 0 writes here.
 __device__ inline bool rs_start(RsCls& S, const PropDev& d, const RsDev& D,
@@ -166,7 +191,6 @@ __device__ inline bool rs_start(RsCls& S, const PropDev& d, const RsDev& D,
   z.s_int = d.inv_perm[ti.s_st - 1];
   z.dt = ti.dt;
   z.counter = 1;
-  z.th_c = __longlong_as_double(0x7ff8000000000000ULL);
   const double k_vec = sqrt(d.mass * 2.0 * ti.e_coll);
   const double l_orb = sqrt(ti.l_real * (ti.l_real + 1.0));
   if (l_orb / k_vec > ti.r_start) {
@@ -227,7 +251,7 @@ __device__ inline SplineAt rs_spline(const double* Rg, const double* ih, int nR,
   return s;
 }
 
-// A trajectory handed over by the lockstep engine (thread 0): its state at the start of an
+// A trajectory handed over by the lockstep engine (one thread): its state at the start of an
 // RK4 step or before its closing evaluation.
 __device__ inline void rs_resume(RsCls& S, const PropDev& d, const RsResume& r,
                                  const mqct_traj_init_t& ti) {
@@ -250,69 +274,69 @@ __device__ inline void rs_resume(RsCls& S, const PropDev& d, const RsResume& r,
   z.period = r.period;
   z.stage = r.stage;
   z.hint = r.hint;
-  z.th_c = __longlong_as_double(0x7ff8000000000000ULL);
   S = z;
 }
 
-// The stage point's scalars, spline interval and factors, and the knot rows to load
-// (thread 0).
-__device__ inline void rs_point(RsCls& S, const PropDev& d, const double* Rg, const double* ih) {
-  const Cls c = S.CT;
-  if (!(c.th == S.th_c)) {
-    const double st0 = sin(c.th);
-    S.th_c = c.th;
-    S.sin_c = st0;
-    S.is2_c = 1.0 / (st0 * st0);
-  }
-  S.sin_t = S.sin_c;
-  S.inv_s2 = S.is2_c;
-  S.inv_r = 1.0 / c.R;
-  S.dphidt = c.Pphi * S.inv_r * S.inv_r * d.inv_mass * S.inv_s2;
+// Point at R: its spline interval and factors and the knot rows to load (one thread).
+__device__ inline void rs_point(RsCls& S, RsPoint& P, const PropDev& d, const double* Rg,
+                                const double* ih, double R) {
+  P.R = R;
+  P.inv_r = 1.0 / R;
   int hint = S.hint;
-  const SplineAt sp = rs_spline(Rg, ih, d.nR, c.R, &hint);
+  const SplineAt sp = rs_spline(Rg, ih, d.nR, R, &hint);
   S.hint = hint;
-  S.cf[0] = (float)sp.aa;
-  S.cf[1] = (float)sp.bb;
-  S.cf[2] = (float)(sp.cc1 * sp.cc5);
-  S.cf[3] = (float)(sp.cc2 * sp.cc5);
-  S.cf[4] = (float)ih[sp.klo];
-  S.cf[5] = (float)(-sp.cc3 * sp.cc6);
-  S.cf[6] = (float)(sp.cc4 * sp.cc6);
+  P.cf[0] = (float)sp.aa;
+  P.cf[1] = (float)sp.bb;
+  P.cf[2] = (float)(sp.cc1 * sp.cc5);
+  P.cf[3] = (float)(sp.cc2 * sp.cc5);
+  P.cf[4] = (float)ih[sp.klo];
+  P.cf[5] = (float)(-sp.cc3 * sp.cc6);
+  P.cf[6] = (float)(sp.cc4 * sp.cc6);
   const int key = sp.zero ? d.nR - 1 : sp.klo;
-  S.key = key;
-  S.load[0] = S.load[1] = -1;
+  P.key = key;
+  P.load[0] = P.load[1] = -1;
   if (sp.zero) return;
   const int a = key, b = key + 1;
   const int t0 = S.tag[0], t1 = S.tag[1];
   if (t0 == a) {
-    S.lo_buf = 0;
-    if (t1 != b) S.load[1] = b;
+    P.lo_buf = 0;
+    if (t1 != b) P.load[1] = b;
   } else if (t1 == a) {
-    S.lo_buf = 1;
-    if (t0 != b) S.load[0] = b;
+    P.lo_buf = 1;
+    if (t0 != b) P.load[0] = b;
   } else if (t0 == b) {
-    S.lo_buf = 1;
-    S.load[1] = a;
+    P.lo_buf = 1;
+    P.load[1] = a;
   } else if (t1 == b) {
-    S.lo_buf = 0;
-    S.load[0] = a;
+    P.lo_buf = 0;
+    P.load[0] = a;
   } else {
-    S.lo_buf = 0;
-    S.load[0] = a;
-    S.load[1] = b;
+    P.lo_buf = 0;
+    P.load[0] = a;
+    P.load[1] = b;
   }
-  if (S.load[0] >= 0) S.tag[0] = S.load[0];
-  if (S.load[1] >= 0) S.tag[1] = S.load[1];
+  if (P.load[0] >= 0) S.tag[0] = P.load[0];
+  if (P.load[1] >= 0) S.tag[1] = P.load[1];
 }
 
-// After the cluster's sums F, g, pot of a right-hand side (thread 0 of every CTA, the
-// same arithmetic in each): the classical RK4 stage, at the end of a step the stop rules
-// (MQCT_SOURCE_CODES/propagator.f:4011-4050), after the closing evaluation the outputs
-// (rank 0; F = quantum energy and g = norm there, the energy bookkeeping of
-// MQCT_SOURCE_CODES/propagator.f:4182-4343).
-__device__ inline void rs_classical(RsCls& S, const PropDev& d, const RsDev& D,
-                                    const mqct_traj_init_t& ti, const double* e_val, int s_ec,
-                                    int tr, bool rank0, double F, double g, double pot) {
+// dphi/dt at point P of the stage input CT, and R of the point after it (one thread).
+__device__ inline double rs_next_r(const RsCls& S, RsPoint& P, const PropDev& d) {
+  P.dphidt = S.CT.Pphi * P.inv_r * P.inv_r * d.inv_mass * S.inv_s2;
+  const double dR = S.CT.PR * d.inv_mass;
+  if (S.stage < 2) return S.C.R + S.dt * 0.5 * dR;
+  if (S.stage == 2) return S.C.R + S.dt * dR;
+  return S.C.R + S.dt / 6.0 * (S.K1.R + dR + 2.0 * S.K23.R);
+}
+
+// After the cluster's sums F, g, pot of the right-hand side at point P (one thread of every
+// CTA, the same arithmetic in each; Rn is R of the next point): the classical RK4 stage, at the
+// end of a step the stop rules (MQCT_SOURCE_CODES/propagator.f:4011-4050), after the closing
+// evaluation the outputs (rank 0; F = quantum energy and g = norm there, the energy
+// bookkeeping of MQCT_SOURCE_CODES/propagator.f:4182-4343).
+__device__ inline void rs_classical(RsCls& S, const RsPoint& P, double Rn, const PropDev& d,
+                                    const RsDev& D, const mqct_traj_init_t& ti,
+                                    const double* e_val, int s_ec, int tr, bool rank0, double F,
+                                    double g, double pot) {
   const int s = S.stage;
   if (s == 4) {
     if (rank0) {
@@ -334,14 +358,14 @@ __device__ inline void rs_classical(RsCls& S, const PropDev& d, const RsDev& D,
     return;
   }
   const Cls c = S.CT;
-  const double im = d.inv_mass, ir = S.inv_r;
+  const double im = d.inv_mass, ir = P.inv_r;
   const double ir3m = ir * ir * ir * im;
   Cls dc;
   dc.R = c.PR * im;
   dc.PR = -F + c.Pth * c.Pth * ir3m + c.Pphi * c.Pphi * ir3m * S.inv_s2;
   dc.th = 0.0;
   dc.Pth = 0.0;
-  dc.phi = S.dphidt;
+  dc.phi = P.dphidt;
   dc.Pphi = S.sin_t * g;
   const double dt = S.dt, hh = dt * 0.5;
   auto axpy = [](const Cls& a, double h, const Cls& x) {
@@ -355,20 +379,23 @@ __device__ inline void rs_classical(RsCls& S, const PropDev& d, const RsDev& D,
       S.eki = kinetic(S.C, d.mass);
     }
     S.CT = axpy(S.C, hh, dc);
+    S.CT.R = Rn;
     S.stage = 1;
   } else if (s == 1) {
     S.K23 = dc;
     S.CT = axpy(S.C, hh, dc);
+    S.CT.R = Rn;
     S.stage = 2;
   } else if (s == 2) {
     S.K23 = axpy(S.K23, 1.0, dc);
     S.CT = axpy(S.C, dt, dc);
+    S.CT.R = Rn;
     S.stage = 3;
   } else {
     const double h6 = dt / 6.0;
     Cls& cc = S.C;
     const Cls &a1 = S.K1, &a23 = S.K23, &a4 = dc;
-    cc.R += h6 * (a1.R + a4.R + 2.0 * a23.R);
+    cc.R = Rn;
     cc.PR += h6 * (a1.PR + a4.PR + 2.0 * a23.PR);
     cc.th += h6 * (a1.th + a4.th + 2.0 * a23.th);
     cc.Pth += h6 * (a1.Pth + a4.Pth + 2.0 * a23.Pth);
@@ -413,9 +440,10 @@ __device__ __forceinline__ void rs_wait() {
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// Phases e^{-iEt} = (cos E t, -sin E t) of the energy classes at time t.
-__device__ inline void rs_phases(float2* ph, const double* ev, int n_e, double t) {
-  for (int e = threadIdx.x; e < n_e; e += RS_THREADS) {
+// Phases e^{-iEt} = (cos E t, -sin E t) of the energy classes at time t, by the threads from
+// tid0 on.
+__device__ inline void rs_phases(float2* ph, const double* ev, int n_e, double t, int tid0) {
+  for (int e = (int)threadIdx.x - tid0; e >= 0 && e < n_e; e += RS_BLOCK - tid0) {
     double sn, co;
     sincos(ev[e] * t, &sn, &co);
     ph[e] = make_float2((float)co, (float)(-sn));
@@ -423,12 +451,12 @@ __device__ inline void rs_phases(float2* ph, const double* ev, int n_e, double t
 }
 
 // One cluster of CL CTAs per trajectory at a time; persistent over the device queue.
-__global__ void __launch_bounds__(RS_THREADS, 1) rs_kernel(PropDev d, RsDev D) {
+__global__ void __launch_bounds__(RS_BLOCK, 1) rs_kernel(PropDev d, RsDev D) {
   cg::cluster_group clu = cg::this_cluster();
   const int rank = (int)clu.block_rank();
   const int tid = threadIdx.x;
   extern __shared__ __align__(16) unsigned char rs_sm[];
-  const RsSmem L = rs_layout(D.ns_cap, D.nr_cap, D.n_e, d.nR);
+  const RsSmem L = rs_layout(D.ns_cap, D.nr_cap, D.n_e, d.nR, D.CL);
   float2* KN[2] = {reinterpret_cast<float2*>(rs_sm + L.kn0), reinterpret_cast<float2*>(rs_sm + L.kn1)};
   float* Mp = reinterpret_cast<float*>(rs_sm + L.mp);
   uint16_t* loc = reinterpret_cast<uint16_t*>(rs_sm + L.loc);
@@ -437,16 +465,17 @@ __global__ void __launch_bounds__(RS_THREADS, 1) rs_kernel(PropDev d, RsDev D) {
   float2* AIN[2] = {reinterpret_cast<float2*>(rs_sm + L.ain0), reinterpret_cast<float2*>(rs_sm + L.ain1)};
   float4* HALO[2] = {reinterpret_cast<float4*>(rs_sm + L.halo0), reinterpret_cast<float4*>(rs_sm + L.halo1)};
   float2* bt = reinterpret_cast<float2*>(rs_sm + L.bt);
-  float2* uv = reinterpret_cast<float2*>(rs_sm + L.u);
   float2* PH[2] = {reinterpret_cast<float2*>(rs_sm + L.ph0), reinterpret_cast<float2*>(rs_sm + L.ph1)};
   RsRow* row = reinterpret_cast<RsRow*>(rs_sm + L.rows);
   double* Rg = reinterpret_cast<double*>(rs_sm + L.rg);
   double* ih = reinterpret_cast<double*>(rs_sm + L.ih);
   double* ev = reinterpret_cast<double*>(rs_sm + L.ev);
+  double* part = reinterpret_cast<double*>(rs_sm + L.part);  // [2][CL][RS_WARPS][3]
+  const int warp = tid >> 5, lane = tid & 31;
+  const bool rows = warp < RS_WARPS, classical = warp == RS_WARPS;
   __shared__ RsCls S;
+  __shared__ RsPoint s_pt[2];  // of this right-hand side and the next, by parity
   __shared__ mqct_traj_init_t s_ti;
-  __shared__ double red[3 * RS_WARPS + 3];
-  __shared__ double part[2][RS_MAX_CL][3];
   __shared__ int s_tr, s_ec;
   __shared__ int s_n[RS_MAX_BLK], s_ls0[RS_MAX_BLK], s_lr0[RS_MAX_BLK], s_q0[RS_MAX_BLK];
   // a row's new stage input into the Coriolis neighbour slots (J_+ in .xy, J_- in .zw of
@@ -466,7 +495,7 @@ __global__ void __launch_bounds__(RS_THREADS, 1) rs_kernel(PropDev d, RsDev D) {
   };
   const int e0 = D.rk_b0[rank], nbk = D.rk_b0[rank + 1] - e0;
   const int nr = D.rk_rows[rank], nsl_r = D.rk_slots[rank];
-  for (int e = tid; e < nbk; e += RS_THREADS) {
+  for (int e = tid; e < nbk; e += RS_BLOCK) {
     const int b = D.rk_blk[e0 + e];
     s_n[e] = d.blk_n[b];
     s_ls0[e] = D.rk_ls0[e0 + e];
@@ -474,17 +503,17 @@ __global__ void __launch_bounds__(RS_THREADS, 1) rs_kernel(PropDev d, RsDev D) {
     s_q0[e] = (int)d.blk_slot0[b];
   }
   // slots of the CTA's blocks (the padding slots keep zero knots: no force, unread M)
-  for (int k = tid; k < D.ns_cap; k += RS_THREADS) {
+  for (int k = tid; k < D.ns_cap; k += RS_BLOCK) {
     loc[k] = D.loc[(size_t)rank * D.ns_cap + k];
     KN[0][k] = make_float2(0.f, 0.f);
     KN[1][k] = make_float2(0.f, 0.f);
   }
-  for (int lr = tid; lr < nr; lr += RS_THREADS) row[lr] = D.rows[(size_t)rank * D.nr_cap + lr];
-  for (int k = tid; k < d.nR; k += RS_THREADS) {
+  for (int lr = tid; lr < nr; lr += RS_BLOCK) row[lr] = D.rows[(size_t)rank * D.nr_cap + lr];
+  for (int k = tid; k < d.nR; k += RS_BLOCK) {
     Rg[k] = d.R[k];
     ih[k] = D.ih[k];
   }
-  for (int e = tid; e < D.n_e; e += RS_THREADS) ev[e] = d.e_val[e];
+  for (int e = tid; e < D.n_e; e += RS_BLOCK) ev[e] = d.e_val[e];
   if (tid == 0) {
     S.tag[0] = -1;
     S.tag[1] = -1;
@@ -504,9 +533,13 @@ __global__ void __launch_bounds__(RS_THREADS, 1) rs_kernel(PropDev d, RsDev D) {
       s_ti = D.init[tr];
       if (D.resume) {
         rs_resume(S, d, D.resume[qi], s_ti);
-        rs_point(S, d, Rg, ih);
-      } else if (rs_start(S, d, D, s_ti, tr, rank == 0)) {
-        rs_point(S, d, Rg, ih);
+      } else {
+        rs_start(S, d, D, s_ti, tr, rank == 0);
+      }
+      if (S.stage != 5) {
+        S.sin_t = sin(S.CT.th);
+        S.inv_s2 = 1.0 / (S.sin_t * S.sin_t);
+        rs_point(S, s_pt[rc & 1], d, Rg, ih, S.CT.R);
       }
       s_ec = d.st_e[S.s_int];
     }
@@ -515,7 +548,7 @@ __global__ void __launch_bounds__(RS_THREADS, 1) rs_kernel(PropDev d, RsDev D) {
     {
       float2* a0 = AIN[rc & 1];
       double* amp = D.amp + (size_t)tr * 2 * d.N;
-      for (int lr = tid; lr < nr; lr += RS_THREADS) {
+      for (int lr = tid; lr < nr; lr += RS_BLOCK) {
         const RsRow w = row[lr];
         const double one = w.gi == S.s_int ? 1.0 : 0.0;
         // a handed-over trajectory's amplitudes, its stage input their FP32 rounding (as
@@ -529,89 +562,93 @@ __global__ void __launch_bounds__(RS_THREADS, 1) rs_kernel(PropDev d, RsDev D) {
           amp[d.N + w.ri] = 0.0;
         }
       }
-      if (go) rs_phases(PH[rc & 1], ev, D.n_e, S.tcur);
+      if (go) rs_phases(PH[rc & 1], ev, D.n_e, S.tcur, 0);
     }
     clu.sync();  // the peers read these amplitudes from the first right-hand side on
     if (!go) continue;
-    while (S.stage != 5) {
-      const int s = S.stage, par = rc & 1;
-      const bool zero = S.key == d.nR - 1;  // above the grid: the matrix is zero
-      // knot rows that the stage point's interval needs and the buffers do not hold
-#pragma unroll
-      for (int bsel = 0; bsel < 2; ++bsel) {
-        const int krow = S.load[bsel];
-        if (krow < 0) continue;
-        const float2* src = reinterpret_cast<const float2*>(d.knots) + (int64_t)krow * d.S;
-        float2* dst = KN[bsel];
-        for (int e = 0; e < nbk; ++e) {
-          const int n = s_n[e], nsl = n * (n + 1) / 2;
-          const float2* se = src + s_q0[e];
-          float2* de = dst + s_ls0[e];
-          for (int q = tid; q < nsl; q += RS_THREADS) de[q] = __ldg(se + q);
-        }
-      }
-      // bt = D^* a and u = (J_+ + J_-) a of this CTA's rows (MQCT_SOURCE_CODES/
-      // mqct_eqtns.f:447-464); the neighbours' stage inputs were pushed into halo
+    bool first = true;
+    for (;;) {
+      const int par = rc & 1;
+      const RsPoint& P = s_pt[par];
+      const bool zero = P.key == d.nR - 1;  // above the grid: the matrix is zero
       const float2* ph = PH[par];
       const float2* ain = AIN[par];
       const float4* halo = HALO[par];
-      for (int lr = tid; lr < nr; lr += RS_THREADS) {
-        const RsRow w = row[lr];
-        const float2 a = ain[lr];
-        const float2 p = ph[w.ec];
-        bt[lr] = make_float2(p.x * a.x - p.y * a.y, p.x * a.y + p.y * a.x);
-        const float4 hv = halo[lr];
-        double ur = 0.0, ui = 0.0;
-        if (w.nbp >= 0) {
-          ur += w.cp * (double)hv.x;
-          ui += w.cp * (double)hv.y;
-        }
-        if (w.nbm >= 0) {
-          ur += w.cm * (double)hv.z;
-          ui += w.cm * (double)hv.w;
-        }
-        uv[lr] = make_float2((float)ur, (float)ui);
-      }
-      __syncthreads();
       float force = 0.f;
-      if (!zero) {
-        // every slot of the CTA: M = aa lo + bb hi + c1 lo'' + c2 hi'' into the packed
-        // triangles, M' = (hi - lo)/h + d1 lo'' + d2 hi'' into the force (two slots per
-        // thread and step, 16-byte knot loads; padding slots hold zero knots)
-        const float aa = S.cf[0], bb = S.cf[1], c1 = S.cf[2], c2 = S.cf[3];
-        const float hinv = S.cf[4], d1 = S.cf[5], d2 = S.cf[6];
-        const float2* K0 = KN[S.lo_buf];
-        const float2* K1 = KN[S.lo_buf ^ 1];
-        for (int k = 2 * tid; k < nsl_r; k += 2 * RS_THREADS) {
-          const float4 lo = *reinterpret_cast<const float4*>(K0 + k);
-          const float4 hi = *reinterpret_cast<const float4*>(K1 + k);
-          const uint32_t l2 = *reinterpret_cast<const uint32_t*>(loc + k);
-          const float m0 = aa * lo.x + bb * hi.x + c1 * lo.y + c2 * hi.y;
-          const float md0 = (hi.x - lo.x) * hinv + d1 * lo.y + d2 * hi.y;
-          const float m1 = aa * lo.z + bb * hi.z + c1 * lo.w + c2 * hi.w;
-          const float md1 = (hi.z - lo.z) * hinv + d1 * lo.w + d2 * hi.w;
-          *reinterpret_cast<float2*>(Mp + k) = make_float2(m0, m1);
-          {
-            const int ia = (int)(l2 & 255u), ib = (int)((l2 >> 8) & 255u);
-            const float2 x = bt[ia], z = bt[ib];
-            force += (ia == ib ? md0 : 2.f * md0) * (x.x * z.x + x.y * z.y);
+      if (classical) {
+        // the cluster's sums of the right-hand side before, its classical stage, dphi/dt of
+        // this point, and the next point (none after the closing evaluation)
+        double F = 0.0, G = 0.0, Q = 0.0;
+        if (!first) rs_sums(part + (size_t)(par ^ 1) * D.CL * RS_WARPS * 3, D.CL, F, G, Q);
+        if (lane == 0) {
+          if (!first)
+            rs_classical(S, s_pt[par ^ 1], P.R, d, D, s_ti, ev, s_ec, tr, rank == 0, F, G, Q);
+          const double Rn = rs_next_r(S, s_pt[par], d);
+          if (S.stage != 4) rs_point(S, s_pt[par ^ 1], d, Rg, ih, Rn);
+        }
+        __syncwarp();
+      } else if (rows) {
+        // knot rows that the point's interval needs and the buffers do not hold
+#pragma unroll
+        for (int bsel = 0; bsel < 2; ++bsel) {
+          const int krow = P.load[bsel];
+          if (krow < 0) continue;
+          const float2* src = reinterpret_cast<const float2*>(d.knots) + (int64_t)krow * d.S;
+          float2* dst = KN[bsel];
+          for (int e = 0; e < nbk; ++e) {
+            const int n = s_n[e], nsl = n * (n + 1) / 2;
+            const float2* se = src + s_q0[e];
+            float2* de = dst + s_ls0[e];
+            for (int q = tid; q < nsl; q += RS_THREADS) de[q] = __ldg(se + q);
           }
-          {
-            const int ia = (int)((l2 >> 16) & 255u), ib = (int)(l2 >> 24);
-            const float2 x = bt[ia], z = bt[ib];
-            force += (ia == ib ? md1 : 2.f * md1) * (x.x * z.x + x.y * z.y);
+        }
+        // bt = D^* a of this CTA's rows (MQCT_SOURCE_CODES/mqct_eqtns.f:447-464)
+        for (int lr = tid; lr < nr; lr += RS_THREADS) {
+          const float2 a = ain[lr];
+          const float2 p = ph[row[lr].ec];
+          bt[lr] = make_float2(p.x * a.x - p.y * a.y, p.x * a.y + p.y * a.x);
+        }
+        asm volatile("bar.sync 1, %0;" ::"n"(RS_THREADS) : "memory");  // the row warps
+        if (!zero) {
+          // every slot of the CTA: M = aa lo + bb hi + c1 lo'' + c2 hi'' into the packed
+          // triangles, M' = (hi - lo)/h + d1 lo'' + d2 hi'' into the force (two slots per
+          // thread and step, 16-byte knot loads; padding slots hold zero knots)
+          const float aa = P.cf[0], bb = P.cf[1], c1 = P.cf[2], c2 = P.cf[3];
+          const float hinv = P.cf[4], d1 = P.cf[5], d2 = P.cf[6];
+          const float2* K0 = KN[P.lo_buf];
+          const float2* K1 = KN[P.lo_buf ^ 1];
+          for (int k = 2 * tid; k < nsl_r; k += 2 * RS_THREADS) {
+            const float4 lo = *reinterpret_cast<const float4*>(K0 + k);
+            const float4 hi = *reinterpret_cast<const float4*>(K1 + k);
+            const uint32_t l2 = *reinterpret_cast<const uint32_t*>(loc + k);
+            const float m0 = aa * lo.x + bb * hi.x + c1 * lo.y + c2 * hi.y;
+            const float md0 = (hi.x - lo.x) * hinv + d1 * lo.y + d2 * hi.y;
+            const float m1 = aa * lo.z + bb * hi.z + c1 * lo.w + c2 * hi.w;
+            const float md1 = (hi.z - lo.z) * hinv + d1 * lo.w + d2 * hi.w;
+            *reinterpret_cast<float2*>(Mp + k) = make_float2(m0, m1);
+            {
+              const int ia = (int)(l2 & 255u), ib = (int)((l2 >> 8) & 255u);
+              const float2 x = bt[ia], z = bt[ib];
+              force += (ia == ib ? md0 : 2.f * md0) * (x.x * z.x + x.y * z.y);
+            }
+            {
+              const int ia = (int)((l2 >> 16) & 255u), ib = (int)(l2 >> 24);
+              const float2 x = bt[ia], z = bt[ib];
+              force += (ia == ib ? md1 : 2.f * md1) * (x.x * z.x + x.y * z.y);
+            }
           }
         }
       }
       __syncthreads();
+      const int s = S.stage;
       // rows: y_i = sum_j M_ij bt_j (tpr threads per row, strided parts of the row joined by
       // shuffles within the lane group); then, by the row's first thread, the quadratic
       // forms (F from above, g = Im((D^* u)^+ y), pot = Re(bt^+ y)), the amplitude
       // derivative da = -i (e^{iEt} y + (dphi/2) u) and the row's RK4 update; the closing
       // evaluation forms the quantum energy and the norm in place of F and g
       double f = (double)force, g = 0.0, pt = 0.0;
-      {
-        const double dt = S.dt, dphidt = S.dphidt;
+      if (rows) {
+        const double dt = S.dt, dphidt = P.dphidt;
         float2* aout = AIN[par ^ 1];
         double* amp = D.amp + (size_t)tr * 2 * d.N;
         double fe = 0.0, nn = 0.0;
@@ -620,15 +657,38 @@ __global__ void __launch_bounds__(RS_THREADS, 1) rs_kernel(PropDev d, RsDev D) {
         for (int rb = 0; rb < nr; rb += ng) {  // the same trip count in every lane
           const int lr = rb + grp;
           float yr = 0.f, yi = 0.f;
+          float2 uu = make_float2(0.f, 0.f);  // u: the neighbours' stage inputs are in halo
+          if (lr < nr && sub == 0) {
+            const float4 hv = halo[lr];
+            double ur = 0.0, ui = 0.0;
+            if (row[lr].nbp >= 0) {
+              ur += row[lr].cp * (double)hv.x;
+              ui += row[lr].cp * (double)hv.y;
+            }
+            if (row[lr].nbm >= 0) {
+              ur += row[lr].cm * (double)hv.z;
+              ui += row[lr].cm * (double)hv.w;
+            }
+            uu = make_float2((float)ur, (float)ui);
+          }
           if (lr < nr && !zero) {
             const int ei = row[lr].ent_i;
             const int e = ei >> 8, i = ei & 255;
             const int n = s_n[e];
             const float2* z = bt + s_lr0[e];
             const float* Mb = Mp + s_ls0[e];
-            for (int j = sub; j < n; j += tpr) {
-              const int addr = j <= i ? i * (i + 1) / 2 + j : j * (j + 1) / 2 + i;
-              const float m = Mb[addr];
+            int j = sub;
+            const float* Mi = Mb + i * (i + 1) / 2;
+#pragma unroll 8
+            for (; j <= i; j += tpr) {
+              const float m = Mi[j];
+              const float2 zz = z[j];
+              yr += m * zz.x;
+              yi += m * zz.y;
+            }
+#pragma unroll 8
+            for (; j < n; j += tpr) {
+              const float m = Mb[j * (j + 1) / 2 + i];
               const float2 zz = z[j];
               yr += m * zz.x;
               yi += m * zz.y;
@@ -640,7 +700,7 @@ __global__ void __launch_bounds__(RS_THREADS, 1) rs_kernel(PropDev d, RsDev D) {
           }
           if (lr >= nr || sub != 0) continue;
           const RsRow w = row[lr];
-          const float2 p = ph[w.ec], uu = uv[lr], b2 = bt[lr];
+          const float2 p = ph[w.ec], b2 = bt[lr];
           pt += (double)(b2.x * yr + b2.y * yi);
           if (s == 4) {
             const double2 wv = Y[lr];
@@ -684,32 +744,35 @@ __global__ void __launch_bounds__(RS_THREADS, 1) rs_kernel(PropDev d, RsDev D) {
           g = nn;
         }
       }
-      // this CTA's parts (warp sums, then the warps in order by one thread per quantity) into
-      // every CTA of the cluster; the cluster barrier (release / acquire: the parts and the
-      // stage inputs pushed above are visible after it) is split so that the next right-hand
-      // side's phases, whose time is known before the classical step, are formed while the
-      // other CTAs arrive
-      rs_warp_parts(f, g, pt, red);
-      if (tid < 3) {
-        double v = 0.0;
-        for (int i = 0; i < RS_WARPS; ++i) v += red[3 * i + tid];
-        for (int r = 0; r < D.CL; ++r) *clu.map_shared_rank(&part[par][rank][tid], r) = v;
+      // the next right-hand side's phases, beside the rows where there are few
+      if (s != 4)
+        rs_phases(PH[par ^ 1], ev, D.n_e, s < 2 ? S.tcur + 0.5 * S.dt : S.tcur + S.dt,
+                  D.n_e <= 256 ? RS_THREADS : 0);
+      // every row warp's parts into every CTA of the cluster; after the cluster barrier
+      // (release / acquire) they, the stage inputs pushed above and the phases are visible
+      if (rows) {
+        rs_warp_sum3(f, g, pt);
+        if (lane < D.CL) {
+          double* q = clu.map_shared_rank(part, lane) +
+                      ((size_t)(par * D.CL + rank) * RS_WARPS + warp) * 3;
+          q[0] = f;
+          q[1] = g;
+          q[2] = pt;
+        }
+        __syncwarp();
       }
       rs_arrive();
-      if (s != 4) rs_phases(PH[par ^ 1], ev, D.n_e, s < 2 ? S.tcur + 0.5 * S.dt : S.tcur + S.dt);
       rs_wait();
-      if (tid == 0) {
-        double F = 0.0, G = 0.0, P = 0.0;
-        for (int r = 0; r < D.CL; ++r) {
-          F += part[par][r][0];
-          G += part[par][r][1];
-          P += part[par][r][2];
-        }
-        rs_classical(S, d, D, s_ti, ev, s_ec, tr, rank == 0, F, G, P);
-        if (S.stage != 5) rs_point(S, d, Rg, ih);
-      }
       ++rc;
-      __syncthreads();
+      first = false;
+      if (s == 4) break;
+    }
+    // the closing evaluation's sums and the outputs
+    if (classical) {
+      double F, G, Q;
+      rs_sums(part + (size_t)((rc & 1) ^ 1) * D.CL * RS_WARPS * 3, D.CL, F, G, Q);
+      if (lane == 0)
+        rs_classical(S, s_pt[(rc & 1) ^ 1], 0.0, d, D, s_ti, ev, s_ec, tr, rank == 0, F, G, Q);
     }
   }
   clu.sync();  // no CTA leaves while another may still read its shared memory
@@ -797,7 +860,7 @@ static int rs_prepare(RsEngine* e, const PropDev& d, const std::vector<int>& blk
     sp = rs_split(blk_n, c);
     bool fit = true;
     for (const auto& v : sp.blocks) fit = fit && (int)v.size() <= RS_MAX_BLK;
-    smem = rs_layout(sp.ns_cap, sp.nr_cap, d.n_e, d.nR).total;
+    smem = rs_layout(sp.ns_cap, sp.nr_cap, d.n_e, d.nR, c).total;
     if (fit && smem <= room && sp.nr_cap <= 256) {
       CL = c;
       break;
@@ -814,7 +877,7 @@ static int rs_prepare(RsEngine* e, const PropDev& d, const std::vector<int>& blk
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
   cfg.gridDim = dim3(CL, 1, 1);
-  cfg.blockDim = dim3(RS_THREADS, 1, 1);
+  cfg.blockDim = dim3(RS_BLOCK, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.attrs = at;
   cfg.numAttrs = 1;
@@ -959,7 +1022,7 @@ static int rs_launch(RsEngine* e, const PropDev& d, const std::vector<int>& blk_
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
   cfg.gridDim = dim3(ncl * e->CL, 1, 1);
-  cfg.blockDim = dim3(RS_THREADS, 1, 1);
+  cfg.blockDim = dim3(RS_BLOCK, 1, 1);
   cfg.dynamicSmemBytes = e->smem;
   cfg.stream = st;
   cfg.attrs = at;
