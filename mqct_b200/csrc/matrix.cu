@@ -950,12 +950,16 @@ int MatrixPlan::init(const mqct_sys_t* sys, const int32_t* ind_mat, int64_t P_, 
         cg[(size_t)st * cg_ld + m1 + j1] =
             clebsch_gordan(j1, m1, j2, sys->m12[st] - m1, sys->j12[st], sys->m12[st]);
     }
-    // the distinct levels (j, vector) of each rotor and their (level, m) tables
+    // the distinct levels (j, vector) of each rotor and their (level, m) tables, of the channels
+    // that have states: the others' j is unchecked, and may be beyond their rows of ldv values
+    std::vector<char> has_states(sys->n_channels, 0);
+    for (int st = 0; st < n_states; ++st) has_states[sys->indx_chann[st] - 1] = 1;
     auto levels = [&](const int32_t* j, const double* v, std::vector<int>& lm_ch,
                       std::vector<int>& lm_m, std::vector<int>& ch_lm) {
       std::vector<int> rep, first;  // a channel per level, the place of its (level, -j)
-      ch_lm.resize(sys->n_channels);
+      ch_lm.assign(sys->n_channels, 0);
       for (int c = 0; c < sys->n_channels; ++c) {
+        if (!has_states[c]) continue;
         const double* vc = v + (size_t)c * ldv;
         size_t l = 0;
         while (l < rep.size() && !(j[rep[l]] == j[c] &&
@@ -982,7 +986,8 @@ int MatrixPlan::init(const mqct_sys_t* sys, const int32_t* ind_mat, int64_t P_, 
       MQCT_CUDA_TRY(d_ch_lm[r].upload(cl[r], stream));
     }
     t0_J2 = 0;
-    for (int c = 0; c < sys->n_channels; ++c) t0_J2 = std::max(t0_J2, (int)sys->j2[c]);
+    for (int c = 0; c < sys->n_channels; ++c)
+      if (has_states[c]) t0_J2 = std::max(t0_J2, (int)sys->j2[c]);
     MQCT_CUDA_TRY(d_pair_psi.alloc((size_t)t0_n_lm[0] * grid->n_beta * n_gamma +
                                    (size_t)t0_n_lm[1] * t0_nbb * t0_ngg +
                                    (size_t)(2 * t0_J2 + 1) * t0_naa));
