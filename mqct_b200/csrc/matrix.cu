@@ -924,8 +924,12 @@ int MatrixPlan::init(const mqct_sys_t* sys, const int32_t* ind_mat, int64_t P_, 
     st_m[s] = sys->m12[s];
   }
   for (int c = 0; c < sys->n_channels; ++c) ch_j[c] = sys->j1[c];
+  // (channels without states are left out: their j is unchecked)
+  std::vector<char> has_states(sys->n_channels, 0);
+  for (int st = 0; st < n_states; ++st) has_states[st_chan[st]] = 1;
   jmax_basis = 0;
-  for (int c = 0; c < sys->n_channels; ++c) jmax_basis = std::max(jmax_basis, (int)sys->j1[c]);
+  for (int c = 0; c < sys->n_channels; ++c)
+    if (has_states[c]) jmax_basis = std::max(jmax_basis, (int)sys->j1[c]);
   if (sys_type == 4) {
     MQCT_CUDA_TRY(d_dtab.alloc((size_t)dtab_off(jmax_basis + 1) * grid->n_beta));
     MQCT_CUDA_TRY(d_phase.alloc((size_t)(2 * jmax_basis + 1) * n_gamma));
@@ -950,10 +954,8 @@ int MatrixPlan::init(const mqct_sys_t* sys, const int32_t* ind_mat, int64_t P_, 
         cg[(size_t)st * cg_ld + m1 + j1] =
             clebsch_gordan(j1, m1, j2, sys->m12[st] - m1, sys->j12[st], sys->m12[st]);
     }
-    // the distinct levels (j, vector) of each rotor and their (level, m) tables, of the channels
-    // that have states: the others' j is unchecked, and may be beyond their rows of ldv values
-    std::vector<char> has_states(sys->n_channels, 0);
-    for (int st = 0; st < n_states; ++st) has_states[sys->indx_chann[st] - 1] = 1;
+    // the distinct levels (j, vector) of each rotor and their (level, m) tables; a channel without
+    // states may have a j beyond its row of ldv values
     auto levels = [&](const int32_t* j, const double* v, std::vector<int>& lm_ch,
                       std::vector<int>& lm_m, std::vector<int>& ch_lm) {
       std::vector<int> rep, first;  // a channel per level, the place of its (level, -j)

@@ -34,3 +34,14 @@ def test_unused_channel_of_two_rotors(mq, gpu_available, j1, j2):
     out = mq.build_matrix(_with_unused_channel(_two_tops(mq), j1, j2), R, GRID5, pes, mij_cutoff=0.0)
     for a, b in zip(out, ref):
         assert np.array_equal(a, b)
+
+
+def test_unused_channel_of_a_top(mq, gpu_available):
+    """Its j may be beyond the rotor functions' table of factorials."""
+    R, pes = mq.r_grid(12, 5.0, 12.0), syn.site_pes(6, seed=4)
+    top = lambda: mq.CollisionSystem(4, syn.asym_channels(2), **TOP)  # noqa: E731
+    ref = mq.build_matrix(top(), R, (9, 7, 0, 0, 0, 0, 1), pes, mij_cutoff=0.0)
+    out = mq.build_matrix(_with_unused_channel(top(), 80, 0), R, (9, 7, 0, 0, 0, 0, 1), pes,
+                          mij_cutoff=0.0)
+    for a, b in zip(out, ref):
+        assert np.array_equal(a, b)
