@@ -25,6 +25,10 @@ void set_error(const char* fmt, ...);
 // through pinned staging slots and host threads (hostcopy.cu), small ones as one copy on
 // `after`; complete on return either way.  Returns an MQCT_ code.
 int copy_d2h_host(void* dst, const void* src, size_t bytes, cudaStream_t after);
+// Lets launches of the kernel fn ask for all the dynamic shared memory a CTA may have.  The limit
+// belongs to the function, which live plans of several sizes (and threads) share: it is set to
+// the device's largest and never to one plan's need.  Returns an MQCT_ code.
+int allow_max_smem(const void* fn);
 
 #define MQCT_CUDA_TRY(expr)                                                        \
   do {                                                                             \

@@ -818,9 +818,10 @@ int MatrixPlan::tc_init() {
     std::vector<double> ones(t.npad, 1.0);
     MQCT_CUDA_TRY(d_col_scale.upload(ones, stream));
   }
-  for (int f = 0; f < 3; ++f)
-    MQCT_CUDA_TRY(cudaFuncSetAttribute(tc_kernel(precision == MQCT_PREC_F16X3, f == 2, f == 1),
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)t.smem));
+  for (int f = 0; f < 3; ++f) {
+    const int rc = allow_max_smem(tc_kernel(precision == MQCT_PREC_F16X3, f == 2, f == 1));
+    if (rc) return rc;
+  }
   return MQCT_OK;
 }
 

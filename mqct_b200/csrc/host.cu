@@ -126,6 +126,17 @@ static void sym_eig(int n, std::vector<double>& a, std::vector<double>& w,
 // Level (j, ka, kc) is eigenvalue number j + ka - kc in ascending order, the
 // (Ka, Kc) labelling of MQCT_SOURCE_CODES/asym_top.f:139-173.  The eigenvector
 // (components K=-j..j) is signed so its first non-negligible component is > 0.
+int allow_max_smem(const void* fn) {
+  int dev = 0, optin = 0;
+  cudaFuncAttributes fa{};
+  MQCT_CUDA_TRY(cudaGetDevice(&dev));
+  MQCT_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  MQCT_CUDA_TRY(cudaFuncGetAttributes(&fa, fn));
+  MQCT_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     optin - (int)fa.sharedSizeBytes));
+  return MQCT_OK;
+}
+
 int asym_top_level(double A, double B, double C, int j, int ka, int kc, double* energy,
                    double* vec) {
   if (j < 0 || ka < 0 || kc < 0 || ka > j || kc > j) return MQCT_E_ARG;

@@ -845,8 +845,10 @@ static int ls_run_t(LsEngine* e, const PropDev& d, const std::vector<int>& blk_n
   MQCT_ARG_CHECK(max_rounds < ((int64_t)1 << 40), "trajectories without a step bound");
   const size_t smem = ((sizeof(typename Cfg::E) * (size_t)L.tri_cap + 15) & ~size_t(15)) +
                       sizeof(T2) * (size_t)Cfg::G * nbmax;
-  MQCT_CUDA_TRY(cudaFuncSetAttribute(ls_rhs_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem));
+  {
+    const int rc = allow_max_smem((const void*)ls_rhs_kernel<T>);
+    if (rc) return rc;
+  }
   int per_sm = 0;
   MQCT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ls_rhs_kernel<T>,
                                                               Cfg::THREADS, smem));

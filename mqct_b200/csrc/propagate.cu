@@ -1082,9 +1082,7 @@ struct PropPlan {
       at_tol = in->eps;
       at_mintm = in->hmin;
       method = MQCT_INTEG_RK4;
-      MQCT_CUDA_TRY(cudaFuncSetAttribute(kernel_ptr(), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem_bytes()));
-      return MQCT_OK;
+      return allow_max_smem(kernel_ptr());
     }
     if (in->method == MQCT_INTEG_ODEINT || in->method == MQCT_INTEG_BK_INT) {
       MQCT_ARG_CHECK(in->eps > 0.0 && in->hmin >= 0.0, "ODEINT needs eps > 0 and hmin >= 0");
@@ -1099,9 +1097,7 @@ struct PropPlan {
     ode_eps = in->eps;
     ode_hmin = in->hmin;
     if (method == MQCT_INTEG_ODEINT && tpb != PT) return set_shape(PT, 1);
-    MQCT_CUDA_TRY(cudaFuncSetAttribute(kernel_ptr(), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem_bytes()));
-    return MQCT_OK;
+    return allow_max_smem(kernel_ptr());
   }
   size_t tsize() const { return arith == MQCT_PROP_FP32 ? 4 : 8; }
 
@@ -1274,7 +1270,7 @@ struct PropPlan {
 
   // Pass layout for the current shape: consecutive m-blocks whose packed triangles fit
   // the shared memory one CTA of the shape may take (the SM's shared memory divided by
-  // the CTAs per SM); uploads the pass tables and sets the kernel's launch limit.
+  // the CTAs per SM); uploads the pass tables.
   int layout() {
     ns = 1;
     while (ns * tpb < N) ns *= 2;
@@ -1307,8 +1303,8 @@ struct PropPlan {
     MQCT_CUDA_TRY(d_pass_slot0.upload(pass_slot0, stream));
     MQCT_CUDA_TRY(d_blk_mp.upload(blk_mp, stream));
     MQCT_CUDA_TRY(d_blk_pass.upload(blk_pass, stream));
-    MQCT_CUDA_TRY(cudaFuncSetAttribute(kernel_ptr(), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem_bytes()));
+    const int rc = allow_max_smem(kernel_ptr());
+    if (rc) return rc;
     MQCT_CUDA_TRY(cudaStreamSynchronize(stream));
     return MQCT_OK;
   }
