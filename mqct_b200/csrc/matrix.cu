@@ -306,8 +306,9 @@ __global__ void sur_weight_kernel(PesDev pes, int G2, int nR, const double* __re
 // acc[row, i] = sum_alpha w_alpha sum_g2 Re(psi_a^* psi_b)[row, g2] W[g2, i] on the FP64
 // tensor cores (mma.sync m8n8k4 f64): a 128 x 8 NT WC tile per CTA of 4 WC warps, K-chunks of
 // 16 grid points.  The integrand of a same-m pair at an alpha point is w_alpha times the
-// alpha-free product (the e^{i m alpha} phases of the two states cancel); every alpha point
-// is contracted, as a chunk of its own.  Warp w takes rows 32 (w % 4) .. +31 and 8 NT columns
+// alpha-free product (the e^{i m alpha} phases of the two states cancel), the same for every
+// point of the midpoint grid; every alpha point is contracted, by a pass of MMAs over the chunk
+// in shared memory.  Warp w takes rows 32 (w % 4) .. +31 and 8 NT columns
 // from 8 NT (w / 4): 4 x NT MMA tiles of 8 x 8, 8 NT FP64 accumulators per lane.  Fixed
 // summation order: reproducible.
 // What bounds it: the FP64 tensor pipe, as long as forming X keeps out of its way.  The
@@ -315,10 +316,14 @@ __global__ void sur_weight_kernel(PesDev pes, int G2, int nR, const double* __re
 // barriers with the MMA pipe idle: 3 445 us at 33 280 rows x 2 304 points x 300 R (0.33 of the
 // FP64 rate).  Here sixteen lanes read the 16 grid points of one row (four lines a load), the
 // next chunk's products are loaded and formed between the MMAs of this one, into the other of
-// two shared buffers, W arrives by cp.async, and two CTAs of eight warps share an SM: 2 115
-// us.  The pipe is then what the warps wait for, at 0.66 of its nominal rate; m16n8k8 (2 160
-// us), one CTA of sixteen warps on 160 columns (2 217 us) and plain FMAs on 8 x 10 register
-// tiles (3 066 us) were no faster.
+// two shared buffers, W arrives by cp.async, and two CTAs of eight warps share an SM: 2 085
+// us.  The pipe is then what the warps wait for, at 0.64 of its nominal 36.8 TFLOP/s with the
+// padding of rows and columns, 0.58 without; m16n8k8 (2 160 us), one CTA of sixteen warps on 160
+// columns (2 217 us) and plain FMAs on 8 x 10 register tiles (3 066 us) were no faster.
+// With 48 alpha points 66.2 ms, 0.87 of the rate: the chunk is loaded and X formed once, beside
+// the MMAs of its last pass (113.4 ms with both repeated for every point; 82.8 in the earlier
+// form).  The passes are one loop with the barrier at its end: as an inner loop over the alpha
+// points, or with their number a constant, the build without the axis took 2 390 to 2 490 us.
 constexpr int F_TM = 128, F_TK = 16;
 constexpr int F_XLD = F_TK + 4;  // 4 mod 16: an A fragment's 4 rows x 4 points in distinct banks
 __host__ __device__ constexpr int f_wld(int TN) { return (TN + 15) / 16 * 16 + 4; }
@@ -357,7 +362,7 @@ contract_fp64_kernel(int G2, int nR, const int* __restrict__ row_a, const int* _
   const int* pra = row_a + row0 + xr;
   const int* prb = row_b + row0 + xr;
   const int na = n_alpha > 0 ? n_alpha : 1;
-  const int n_vc = (G2 + F_TK - 1) / F_TK * na;    // chunks, each alpha point its own
+  const int n_vc = (G2 + F_TK - 1) / F_TK * na;    // passes over a chunk: one per alpha point
   auto load_w = [&](int ck, int buf) {
     for (int q = tid; q < F_TK * TN; q += THREADS) {
       const int kk = q / TN, cc = q - kk * TN, g = ck * F_TK + kk, col = col0 + cc;
@@ -383,10 +388,12 @@ contract_fp64_kernel(int G2, int nR, const int* __restrict__ row_a, const int* _
   };
   auto form_x = [&](double wa, int h, int buf) {
 #pragma unroll
-    for (int q = 0; q < NX; ++q)
-      Xs[(buf * F_TM + xr + 2 * (NX * h + q)) * F_XLD + xk] = wa * (u[q].x * v[q].x + u[q].y * v[q].y);
+    for (int q = 0; q < NX; ++q)  // (one fused form: the same bits from every tile shape)
+      Xs[(buf * F_TM + xr + 2 * (NX * h + q)) * F_XLD + xk] =
+          wa * fma(u[q].x, v[q].x, u[q].y * v[q].y);
   };
-  auto weight = [&](int al) { return n_alpha > 0 ? __ldg(walpha + al) : 1.0; };
+  // (the midpoint grid's, alike for every alpha point)
+  auto weight = [&]() { return n_alpha > 0 ? __ldg(walpha) : 1.0; };
   auto mma = [&](int ks, int buf) {
     double av[4], bv[NT];
 #pragma unroll
@@ -401,7 +408,7 @@ contract_fp64_kernel(int G2, int nR, const int* __restrict__ row_a, const int* _
   };
   load_w(0, 0);
   {
-    const double wa = weight(0);
+    const double wa = weight();
 #pragma unroll
     for (int h = 0; h < 4; ++h) {
       load_x(0, h);
@@ -410,18 +417,18 @@ contract_fp64_kernel(int G2, int nR, const int* __restrict__ row_a, const int* _
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
-  int ck = 0, al = 0;
+  int ck = 0, al = 0, cur = 0;
   for (int vc = 0; vc < n_vc; ++vc) {
-    const int cur = vc & 1, nxt = cur ^ 1;
-    const bool more = vc + 1 < n_vc;
+    const int nxt = cur ^ 1;
     if (++al == na) {
       al = 0;
       ++ck;
     }
+    const bool more = vc + 1 < n_vc && al == 0;    // the chunk's last pass, and another follows
     double wa = 1.0;
     if (more) {
       load_w(ck, nxt);
-      wa = weight(al);
+      wa = weight();
     }
 #pragma unroll
     for (int h = 0; h < 4; ++h) {
@@ -429,8 +436,11 @@ contract_fp64_kernel(int G2, int nR, const int* __restrict__ row_a, const int* _
       mma(h, cur);
       if (more) form_x(wa, h, nxt);
     }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();
+    if (more) {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      __syncthreads();
+      cur = nxt;
+    }
   }
 #pragma unroll
   for (int a = 0; a < 4; ++a) {
@@ -447,7 +457,7 @@ contract_fp64_kernel(int G2, int nR, const int* __restrict__ row_a, const int* _
 
 // Tile shapes: (NT, WC) with the clocks of one chunk measured on a B200 with the SM's places
 // (4 / WC CTAs) filled; the shape with the least waves x clocks is taken.  The wide shapes
-// win where there are many tiles (2 115 us for 260 row tiles x 300 R against 2 480 with 32
+// win where there are many tiles (2 085 us for 260 row tiles x 300 R against 2 470 with 32
 // columns), 32 columns by sixteen warps where a build has too few tiles to fill the GPU (19
 // row tiles x 201 R x 576 points: 53 us against 80 with 64 columns; before 146).
 struct FpShape {
