@@ -818,11 +818,25 @@ int MatrixPlan::tc_init() {
     std::vector<double> ones(t.npad, 1.0);
     MQCT_CUDA_TRY(d_col_scale.upload(ones, stream));
   }
-  for (int f = 0; f < 3; ++f) {
-    const int rc = allow_max_smem(tc_kernel(precision == MQCT_PREC_F16X3, f == 2, f == 1));
-    if (rc) return rc;
-  }
-  return MQCT_OK;
+  return tc_pick();
+}
+
+// The kernel form for the plan's settings, with its shared-memory limit (only a form that the plan
+// launches is loaded: the first one of a process takes most of a millisecond).
+int MatrixPlan::tc_pick() {
+  TcInfo& t = *tc;
+  const int n_alpha_it = std::max(1, n_alpha);
+  const bool multi = n_alpha_it > t.slices_per_drain;
+  // sixteen epilogue warps when a K-chunk has several accumulation groups (the drains then
+  // dominate: the as-written alpha grid), eight when it has one (the drain of a chunk then
+  // alternates with its X production, and eight warps with more registers are faster)
+  const bool many = t.pe_force ? t.pe_force == 16 : multi;
+  t.pe_warps = many ? 16 : 8;
+  const void* fn = tc_kernel(precision == MQCT_PREC_F16X3, many, multi);
+  if (fn == t.fn) return MQCT_OK;
+  const int rc = allow_max_smem(fn);
+  if (rc == MQCT_OK) t.fn = fn;
+  return rc;
 }
 
 int MatrixPlan::tc_execute() {
@@ -886,17 +900,12 @@ int MatrixPlan::tc_execute() {
   a.ldp = tc_ldp;
   a.status = d_status.p;
   int grid = std::min(a.n_units, t.n_sm);
-  // sixteen epilogue warps when a K-chunk has several accumulation groups (the drains then
-  // dominate: the as-written alpha grid), eight when it has one (the drain of a chunk then
-  // alternates with its X production, and eight warps with more registers are faster)
-  const bool many = t.pe_force ? t.pe_force == 16
-                               : (a.n_alpha_it + a.slices_per_drain - 1) / a.slices_per_drain >= 2;
-  t.pe_warps = many ? 16 : 8;
-  const bool multi = a.n_alpha_it > a.slices_per_drain;
+  const int rc = tc_pick();
+  if (rc) return rc;
   void* args[] = {&a};
-  MQCT_CUDA_TRY(cudaLaunchKernel(tc_kernel(f16, many, multi), dim3(grid),
-                                 dim3(many ? TcShape<16>::THREADS : TcShape<8>::THREADS), args,
-                                 t.smem, stream));
+  MQCT_CUDA_TRY(cudaLaunchKernel(t.fn, dim3(grid),
+                                 dim3(t.pe_warps == 16 ? TcShape<16>::THREADS : TcShape<8>::THREADS),
+                                 args, t.smem, stream));
   MQCT_CUDA_TRY(cudaGetLastError());
   return MQCT_OK;
 }

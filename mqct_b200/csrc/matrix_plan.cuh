@@ -28,6 +28,7 @@ struct TcInfo {
   int slices_per_drain = 1;                            // alpha points per drain
   bool alpha_uniform = true;                           // all alpha weights equal
   int pe_warps = 8;                                    // epilogue warps of the last launch
+  const void* fn = nullptr;                            // kernel form of the last launch
   int pe_force = 0;                                    // 8 or 16 (tuned or set), 0: by rule
   float pe_tune_ms[2] = {0.f, 0.f};                    // contraction ms with 8 and 16
   uint32_t b_stage = 0, psi_stage = 0;                 // bytes of one such buffer
@@ -114,6 +115,7 @@ struct MatrixPlan {
   DevBuf<int> d_status;
   std::unique_ptr<TcInfo> tc;
   int tc_init();
+  int tc_pick();
   int tc_execute();
   int tc_check_status();
   int error_report(const double* d_mat, mqct_err_report_t* err);
