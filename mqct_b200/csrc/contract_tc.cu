@@ -59,6 +59,7 @@
 // 16 B core matrices, K-adjacent core matrices LBO apart, 8-row groups SBO =
 // 128 B apart.  Every mbarrier wait is bounded; on timeout the CTA records an
 // error code, drains, frees its TMEM and returns.
+#include <cfloat>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -213,6 +214,16 @@ __device__ __forceinline__ F32x2 pack2(uint32_t a, uint32_t b) {
 __device__ __forceinline__ void two_sum(F32x2& S, F32x2& E, F32x2 x) {
   const F32x2 t = add2(S, x), z = sub2(t, S);
   E = add2(E, add2(sub2(S, sub2(t, z)), sub2(x, z)));
+  S = t;
+}
+// E back into S, what does not fit S's 24 bits left in E.  (An infinite S has a NaN in E: fmaxf
+// takes the number, and S stays.)
+__device__ __forceinline__ void fold(F32x2& S, F32x2& E) {
+  const F32x2 e = pack2(
+      __float_as_uint(fmaxf(__uint_as_float((uint32_t)E.v), -FLT_MAX)),
+      __float_as_uint(fmaxf(__uint_as_float((uint32_t)(E.v >> 32)), -FLT_MAX)));
+  const F32x2 t = add2(S, e);
+  E = sub2(e, sub2(t, S));
   S = t;
 }
 // S + E in FP64; an infinite or NaN sum stays what it is.
@@ -656,13 +667,9 @@ __global__ void __launch_bounds__(TcShape<PE>::THREADS, 1) tc_contract_kernel(Tc
             }
           }
         }
-        if (kMulti && a.n_alpha_it > a.slices_per_drain) {  // E stays below an ulp of S
+        if (kMulti && a.n_alpha_it > a.slices_per_drain) {  // E goes back below an ulp of S
 #pragma unroll
-          for (int i = 0; i < TC_NCH_MAX / 2; ++i) {
-            const F32x2 t = add2(S[i], E[i]);
-            E[i] = sub2(E[i], sub2(t, S[i]));
-            S[i] = t;
-          }
+          for (int i = 0; i < TC_NCH_MAX / 2; ++i) fold(S[i], E[i]);
         }
         if (ok && !ahead && c + 1 < c1 && !produce(kc + 1, ka + 1)) ok = false;
       }
