@@ -502,6 +502,15 @@ int mqct_prop_plan_shape(const mqct_prop_plan* plan, int32_t* threads, int32_t* 
 #define MQCT_ENGINE_LOCKSTEP_TAIL 4
 int mqct_prop_plan_set_engine(mqct_prop_plan* plan, int32_t engine);
 int mqct_prop_plan_engine(const mqct_prop_plan* plan, int32_t* engine, int64_t* rounds);
+/* MQCT_ENGINE_PER_TRAJECTORY has two kernels: FP64 runs with fixed RK4 steps and without
+ * SAVE_TRAJECT records take a form that keeps a spline interval's tables in one SM's shared
+ * memory where they fit (at most 704 states, 32 bytes per element of the m-blocks' squares), in
+ * standard and AT mode, with or without CS; all other runs take the general form.  The two differ
+ * in the order of their sums, so a run with records and the same run without agree to rounding,
+ * not to the last bit.  It is the faster kernel for FP64 batches of any size whose tables fit, also
+ * for those of at least 4096 trajectories, which MQCT_ENGINE_AUTO gives to the lockstep engine.
+ * mqct_prop_plan_tune times the launch shapes of the general form.  *one_sm: 1 if the plan's last run took the one-SM form. */
+int mqct_prop_plan_one_sm(const mqct_prop_plan* plan, int32_t* one_sm);
 /* Cluster size of the resident engine: 0 (default) eight CTAs for a batch that the
  * clusters of eight hold at once, else the smallest of 2..8 CTAs whose shared memory holds
  * the tables; or a size in 2..8 (used when the tables fit it).  mqct_prop_plan_cluster

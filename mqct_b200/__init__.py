@@ -793,6 +793,13 @@ class PropagationPlan:
         check(lib().mqct_prop_plan_handed(self.h, C.byref(n)))
         return int(n.value)
 
+    def one_sm(self):
+        """Whether the last run took the one-SM form of the per-trajectory kernel
+        (mqct_prop_plan_one_sm)."""
+        n = C.c_int32()
+        check(lib().mqct_prop_plan_one_sm(self.h, C.byref(n)))
+        return bool(n.value)
+
     def engine(self):
         """(engine of the last run, lockstep rounds of the last run or 0)."""
         e, r = C.c_int32(), C.c_int64()

@@ -100,6 +100,7 @@ EXPORTS = [
     "mqct_prop_plan_destroy", "mqct_prop_plan_set_coupled_states", "mqct_prop_plan_tune",
     "mqct_prop_plan_shape", "mqct_prop_plan_set_engine", "mqct_prop_plan_engine",
     "mqct_prop_plan_set_cluster", "mqct_prop_plan_cluster", "mqct_prop_plan_handed",
+    "mqct_prop_plan_one_sm",
     "mqct_asym_top_level", "mqct_count_states", "mqct_enumerate_states", "mqct_count_pairs",
     "mqct_fill_ind_mat", "mqct_count_states_identical", "mqct_enumerate_states_identical",
     "mqct_count_pairs_identical", "mqct_fill_ind_mat_identical", "mqct_r_grid", "mqct_write_mtrx_uf", "mqct_read_mtrx_uf_header",
@@ -184,6 +185,7 @@ def lib():
     L.mqct_prop_plan_engine.argtypes = [vp, C.POINTER(C.c_int32), C.POINTER(C.c_int64)]
     L.mqct_prop_plan_set_cluster.argtypes = [vp, C.c_int32]
     L.mqct_prop_plan_handed.argtypes = [vp, C.POINTER(C.c_int32)]
+    L.mqct_prop_plan_one_sm.argtypes = [vp, C.POINTER(C.c_int32)]
     L.mqct_prop_plan_cluster.argtypes = [vp, C.POINTER(C.c_int32), C.POINTER(C.c_int32)]
     L.mqct_expansion_plan_create.argtypes = [C.POINTER(Sys), i32p, C.c_int64, f64p, C.c_int32,
                                              C.c_int32, i32p, C.c_double, C.c_double, C.c_double,

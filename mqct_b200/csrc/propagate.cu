@@ -1031,6 +1031,7 @@ struct PropPlan {
   // engine choice (MQCT_ENGINE_*), the engine of the last run and the lockstep engine
   int engine = MQCT_ENGINE_AUTO;
   int last_engine = 0;
+  bool last_one_sm = false;  // the last per-trajectory run took the one-SM form
   LsEngine* ls = nullptr;
   RsEngine* rs = nullptr;
   OcEngine* oc = nullptr;
@@ -1383,9 +1384,15 @@ struct PropPlan {
   double bytes_per_step() const { return 4.0 * (double)S * (4.0 * tsize() + 4.0); }
 
   // FP64 runs with fixed RK4 steps and no SAVE_TRAJECT records take the one-SM form of the
-  // per-trajectory kernel (onecta.cu) where the tables fit it, whatever the batch: 400 steps of
-  // 48 trajectories (165 states) take 2.5 ms against 8.0, of 600 12.4 against 30.5; tables of 35
-  // states and 2 000 trajectories 6.3 against 43.9; no size that fits was slower.
+  // per-trajectory kernel (onecta.cu) where the tables fit it, whatever the number of trajectories:
+  // 400 steps of 48 (165 states) take 2.5 ms against 8.0, of 600 12.4 against 30.5; tables of 35
+  // states and 2 000 trajectories 6.3 against 43.9.  No size that fits was slower, with many
+  // energy classes neither, whose phases one warp forms (400 states, 20 and 400 classes: 200 steps
+  // of 48 trajectories 2.02 and 2.29 ms against 4.92 and 4.95, of 600 9.96 and 11.3 against 23.7
+  // and 24.7).  It serves the runs that come to the per-trajectory kernel: with MQCT_ENGINE_AUTO
+  // standard batches from kLockstepMinBatch on go to the lockstep engine before it is asked, a line
+  // measured on tables that do not fit here (144 states, 100 steps of 4 096 trajectories: 8.3 ms
+  // here with MQCT_ENGINE_PER_TRAJECTORY, 143 in lockstep).
   bool use_one_cta(bool records) {
     if (arith != MQCT_PROP_FP64 || records || method != MQCT_INTEG_RK4 || at_adapt) return false;
     if (!oc) oc = oc_create();
@@ -1397,7 +1404,8 @@ struct PropPlan {
              int64_t* n_rec = nullptr) {
     MQCT_ARG_CHECK(n_traj > 0 && n_traj < (1 << 30), "n_traj out of range");
     last_engine = MQCT_ENGINE_PER_TRAJECTORY;
-    if (use_one_cta(rec != nullptr))
+    last_one_sm = use_one_cta(rec != nullptr);
+    if (last_one_sm)
       return oc_run(oc, dev_view(mode), n_sm, stream, ev0, ev1, d_init_p, (int)n_traj, amp, cls,
                     diag);
     return launch_general(d_init_p, n_traj, mode, amp, cls, diag, rec, rec_cap, n_rec);
@@ -1793,6 +1801,13 @@ int mqct_prop_plan_set_engine(mqct_prop_plan* plan, int32_t engine) {
                      engine == MQCT_ENGINE_LOCKSTEP_TAIL,
                  "unknown engine %d", engine);
   reinterpret_cast<PropPlan*>(plan)->engine = engine;
+  return MQCT_OK;
+}
+
+int mqct_prop_plan_one_sm(const mqct_prop_plan* plan, int32_t* one_sm) {
+  MQCT_ARG_CHECK(plan && one_sm, "null argument");
+  const PropPlan* p = reinterpret_cast<const PropPlan*>(plan);
+  *one_sm = p->last_engine == MQCT_ENGINE_PER_TRAJECTORY && p->last_one_sm ? 1 : 0;
   return MQCT_OK;
 }
 
