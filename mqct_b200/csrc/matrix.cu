@@ -2193,6 +2193,12 @@ __global__ void ex_scatter_kernel(int64_t P, const int* __restrict__ ind_mat,
   order[atomicAdd(count + c, 1)] = (int)k;
 }
 
+// The pairs in their own order, every step-th place.
+__global__ void ex_order_kernel(int64_t P, int step, int* __restrict__ order) {
+  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k < P) order[k * step] = (int)k;
+}
+
 // The groups' rows of FK and rotor factors.
 __global__ void ex_group_kernel(int n_groups, int G, const int* __restrict__ order,
                                 const int* __restrict__ ind_mat, const int* __restrict__ st_chan,
@@ -2245,7 +2251,7 @@ expansion_kernel(int n_groups, FinGrid g, ExpCoef ex, const int* __restrict__ or
   auto look = [&](int i) {
     if (i >= n_groups) return;
 #pragma unroll
-    for (int q = 0; q < G; ++q) n_k[q] = order[i * G + q];
+    for (int q = 0; q < G; ++q) n_k[q] = order[(unsigned)i * G + q];
     if (!ex.A) n_g = grp[i];
   };
   look(gi);
@@ -2447,12 +2453,22 @@ struct ExpansionPlan {
     int dev = 0, n_sm = 0;
     MQCT_CUDA_TRY(cudaGetDevice(&dev));
     MQCT_CUDA_TRY(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
-    const int G = ex_group(nR, P, n_sm);
+    int G = ex_group(nR, P, n_sm);
     const int64_t nc2 = (int64_t)n_ch * n_ch;
-    MQCT_ARG_CHECK(nc2 < ((int64_t)1 << 31) - 1, "%d channels beyond the expansion build", n_ch);
     // places: the pairs, and at most G - 1 empty ones per channel pair that has pairs
     const int64_t cap = P + (G - 1) * std::min<int64_t>(P, nc2);
-    MQCT_ARG_CHECK(cap < ((int64_t)1 << 31), "too many pairs");
+    // (beyond 32-bit counts the pairs keep their order: stored coefficients in full groups, which
+    // may then differ in their zeros, the others one pair a group)
+    if (nc2 >= ((int64_t)1 << 31) - 1 || cap >= ((int64_t)1 << 31)) {
+      if (!a_stored) G = std::min(G, 2);
+      const int step = a_stored ? 1 : G;
+      n_groups = (int)((P * step + G - 1) / G);
+      MQCT_CUDA_TRY(d_order.alloc((size_t)n_groups * G));
+      MQCT_CUDA_TRY(cudaMemsetAsync(d_order.p, 0xff, sizeof(int) * (size_t)n_groups * G, st));
+      ex_order_kernel<<<(unsigned)((P + 255) / 256), 256, 0, st>>>(P, step, d_order.p);
+      MQCT_CUDA_TRY(cudaGetLastError());
+      return groups_and_shape(G, n_sm);
+    }
     DevBuf<int> cnt;
     MQCT_CUDA_TRY(cnt.alloc((size_t)nc2 + 1));
     MQCT_CUDA_TRY(d_order.alloc((size_t)cap));
@@ -2467,13 +2483,16 @@ struct ExpansionPlan {
     MQCT_CUDA_TRY(cudaGetLastError());
     MQCT_CUDA_TRY(cudaStreamSynchronize(st));  // total; the counts are released on return
     n_groups = total / G;
+    return groups_and_shape(G, n_sm);
+  }
+  int groups_and_shape(int G, int n_sm) {
     if (!a_stored) {
       MQCT_CUDA_TRY(d_grp.alloc((size_t)n_groups));
       ex_group_kernel<<<(unsigned)((n_groups + 255) / 256), 256, 0, st>>>(
           n_groups, G, d_order.p, d_ind.p, d_chan.p, d_j1.p, d_j2.p, n_ch, n_terms, d_grp.p);
       MQCT_CUDA_TRY(cudaGetLastError());
-      MQCT_CUDA_TRY(cudaStreamSynchronize(st));
     }
+    MQCT_CUDA_TRY(cudaStreamSynchronize(st));  // the set-up buffers are released on return
     MQCT_CUDA_TRY(d_queue.alloc(2));
     MQCT_CUDA_TRY(cudaMemsetAsync(d_queue.p, 0, 2 * sizeof(int), st));
     return expansion_shape(n_groups, nR, n_terms, G, n_sm, &fin);
