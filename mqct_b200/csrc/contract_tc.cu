@@ -156,8 +156,8 @@ __device__ __forceinline__ void mma_group(uint32_t td, uint32_t ad0, uint64_t bd
     }
   }
 }
-// 8 consecutive TMEM columns of this warp's lane quarter (one 32-bit value per lane each);
-// the values are valid after tmem_wait().
+// 16, 8 or 4 consecutive TMEM columns of this warp's lane quarter (one 32-bit value per lane
+// each); the values are valid after tmem_wait().
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,"
@@ -390,7 +390,7 @@ __global__ void tc_psiimage_kernel(const double2* __restrict__ psi, int G2, int 
 
 // ---------------------------------------------------------------- main kernel
 struct TcArgs {
-  int n_units, n_parts, n_ks, n_chunks, chunks_per_ks, n_alpha_it, nbmax;
+  int n_units, n_parts, n_ks, n_chunks, chunks_per_ks, n_alpha_it;
   int slices_per_drain;           // alpha points accumulated in FP32 between two drains
   int nbuf;                       // B / basis-slice buffers (1 or 2)
   uint32_t b_stage, psi_stage;    // bytes of one B / basis-slice buffer
@@ -403,7 +403,7 @@ struct TcArgs {
   const int* rowb;
   const float2* psi_img;
   const unsigned short* b_img;    // hi/lo planes of W, BF16 or F16 bits, per column part
-  const double* walpha;           // alpha weights (n_alpha_it), or null (weight 1)
+  const double* walpha;           // the weight of every alpha point, or null (weight 1)
   const double* col_scale;        // per radial column: factor applied to the FP64 sums
   double* part;                   // n_ks x n_rows x ldp FP64 sums
   int64_t part_stride;
@@ -737,7 +737,7 @@ int MatrixPlan::tc_init() {
     c += w;
   }
   t.n_chunks = (G2 + TC_KC - 1) / TC_KC;
-  std::vector<int> row0(h_block_row0), nb(h_block_n), bm(h_block_m);
+  std::vector<int> row0(h_block_row0), nb(h_block_n);
   t.n_blocks = (int)row0.size();
   t.nbmax = 0;
   std::vector<int64_t> off(t.n_blocks);
@@ -747,7 +747,7 @@ int MatrixPlan::tc_init() {
     acc += (int64_t)nb[b] * t.n_chunks * TC_PSI_LD;
     t.nbmax = std::max(t.nbmax, nb[b]);
   }
-  // shared memory: B buffers, basis-slice buffers, two A stages, barriers
+  // shared memory: B buffers, basis-slice buffers, barriers
   int ncmax = 0;
   for (int p = 0; p < t.n_parts; ++p) ncmax = std::max(ncmax, t.part_nc[p]);
   auto up = [](size_t x) { return (x + 1023) & ~size_t(1023); };
@@ -765,16 +765,10 @@ int MatrixPlan::tc_init() {
   t.smem = std::max(t.smem, (size_t)dev_smem / 2 + 1024);
   MQCT_CUDA_TRY(t.blk_row0.upload(row0, stream));
   MQCT_CUDA_TRY(t.blk_n.upload(nb, stream));
-  MQCT_CUDA_TRY(t.blk_m.upload(bm, stream));
   MQCT_CUDA_TRY(t.blk_img_off.upload(off, stream));
-  if (n_alpha > 0) MQCT_CUDA_TRY(t.walpha.upload(h_walpha, stream));
   // alpha points per drain: 2 keeps the drains under the MMA time.  The weight is applied to the
   // sums: it is the same for every point of the midpoint grid, the only alpha grid there is.
-  t.alpha_uniform = true;
-  for (int i = 1; i < n_alpha; ++i)
-    if (h_walpha[i] != h_walpha[0]) t.alpha_uniform = false;
-  MQCT_ARG_CHECK(t.alpha_uniform, "the tcgen05 contraction needs equal alpha weights");
-  t.slices_per_drain = (n_alpha > 1 && t.alpha_uniform) ? 2 : 1;
+  t.slices_per_drain = n_alpha > 1 ? 2 : 1;
   // K ranges: split the chunks only to fill the last wave of units, or the SMs when the units of
   // one range are fewer (the FP64 sums of every range are written once and added by the
   // finalize).  The cost of ks ranges, in accumulation groups: a chunk's groups and its X, and 15
@@ -887,7 +881,6 @@ int MatrixPlan::tc_execute() {
   a.chunks_per_ks = t.chunks_per_split;
   a.n_alpha_it = n_alpha > 0 ? n_alpha : 1;
   a.slices_per_drain = std::max(1, std::min(t.slices_per_drain, a.n_alpha_it));
-  a.nbmax = t.nbmax;
   a.nbuf = t.nbuf;
   a.b_stage = t.b_stage;
   a.psi_stage = t.psi_stage;
@@ -900,7 +893,7 @@ int MatrixPlan::tc_execute() {
   a.rowb = d_rowb.p;
   a.psi_img = d_psi32.p;
   a.b_img = d_bimg.p;
-  a.walpha = n_alpha > 0 ? t.walpha.p : nullptr;
+  a.walpha = n_alpha > 0 ? d_walpha.p : nullptr;
   a.col_scale = d_col_scale.p;
   a.part = d_part.p;
   a.part_stride = (int64_t)n_rows * tc_ldp;

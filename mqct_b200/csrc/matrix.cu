@@ -53,10 +53,6 @@ static int upload_logfact() {
 // (alpha2, beta1, beta2, gamma1, gamma2), gamma2 fastest; alpha1 = 0 with the
 // analytic factor 2 pi in the weights (MQCT_SOURCE_CODES/pot_comp.f:3663-3721).
 struct Type0Dev {
-  const int* ch_j2;        // per channel
-  const double* vec2;      // per channel, stride ldv
-  const double* cg;        // per state: CG(j1 m1 j2 m12-m1 | j12 m12) at [m1 + j1], stride cg_ld
-  int cg_ld;
   const double* beta2;
   const double* alpha2;
   const double* gamma2;
@@ -820,7 +816,6 @@ int MatrixPlan::init(const mqct_sys_t* sys, const int32_t* ind_mat, int64_t P_, 
     block_row0.push_back((int)row_state.size());
     h_block_row0.push_back((int)row_state.size());
     h_block_n.push_back((int)kv.second.size());
-    h_block_m.push_back(kv.first);
     for (size_t l = 0; l < kv.second.size(); ++l) {
       state_block[kv.second[l]] = (int)block_row0.size() - 1;
       state_local[kv.second[l]] = (int)l;
@@ -838,7 +833,7 @@ int MatrixPlan::init(const mqct_sys_t* sys, const int32_t* ind_mat, int64_t P_, 
                    (long long)k + 1);
     ks[state_block[a]].push_back(k);
   }
-  std::vector<int> rowa, rowb, rowm, k2r(P);
+  std::vector<int> rowa, rowb, k2r(P);
   std::vector<int> tile_block;
   for (size_t blk = 0; blk < ks.size(); ++blk) {
     if (ks[blk].empty()) continue;
@@ -848,12 +843,10 @@ int MatrixPlan::init(const mqct_sys_t* sys, const int32_t* ind_mat, int64_t P_, 
       k2r[k] = (int)rowa.size();
       rowa.push_back(block_row0[blk] + state_local[a]);
       rowb.push_back(block_row0[blk] + state_local[b]);
-      rowm.push_back(sys->m12[a]);
     }
     while ((rowa.size() - start) % 128) {  // pad to whole tiles; padded rows are never read back
       rowa.push_back(rowa[start]);
       rowb.push_back(rowb[start]);
-      rowm.push_back(rowm[start]);
     }
     for (size_t t = start; t < rowa.size(); t += 128) tile_block.push_back((int)blk);
   }
@@ -913,10 +906,7 @@ int MatrixPlan::init(const mqct_sys_t* sys, const int32_t* ind_mat, int64_t P_, 
       n_alpha = grid->n_alpha;
       std::vector<double> wa(n_alpha);
       for (int i = 0; i < n_alpha; ++i) wa[i] = aa.w[i] * aa.half;
-      MQCT_CUDA_TRY(d_alpha.upload(aa.x, stream));
       MQCT_CUDA_TRY(d_walpha.upload(wa, stream));
-      h_alpha = aa.x;
-      h_walpha = wa;
     }
   }
   h_beta = ab.x;
@@ -1016,7 +1006,6 @@ int MatrixPlan::init(const mqct_sys_t* sys, const int32_t* ind_mat, int64_t P_, 
   }
   MQCT_CUDA_TRY(d_rowa.upload(rowa, stream));
   MQCT_CUDA_TRY(d_rowb.upload(rowb, stream));
-  MQCT_CUDA_TRY(d_rowm.upload(rowm, stream));
   MQCT_CUDA_TRY(d_k2r.upload(k2r, stream));
   h_rowa = rowa;
   h_rowb = rowb;
@@ -1092,10 +1081,11 @@ int MatrixPlan::init(const mqct_sys_t* sys, const int32_t* ind_mat, int64_t P_, 
 int MatrixPlan::upload_site_terms(const mqct_pes_t* pes) {
   pes_sites = false;
   if (pes->kind != MQCT_PES_SITES1 && pes->kind != MQCT_PES_SITES2) return MQCT_OK;
-  // The FP64 form of a rotor + atom build keeps the general kernel: its last bits are those that
-  // FP32 trajectory tables are rounded from (the site kernel moves 216 of 9.6 million elements
-  // by an FP32 unit, and the amplitudes of 48 trajectories by 1e-8), and the surface is 3% of
-  // its time (69 against 49 us of a 2 300 us build).
+  // The FP64 form of a rotor + atom build keeps the general kernel.  Neither is the more accurate
+  // (median error of a value against 64-bit-significand arithmetic 5.4e-16 general, 4.8e-16 site
+  // kernel; 1% above 6.6e-15 and 6.7e-15), so nothing is gained by moving the last bits that FP32
+  // trajectory tables are rounded from (216 of 9.6 million elements by an FP32 unit), and the
+  // surface is 3% of the build (69 against 49 us of 2 300).
   if (precision == MQCT_PREC_FP64 && sys_type != 0) return MQCT_OK;
   const bool two = pes->kind == MQCT_PES_SITES2;
   const int per = two ? 7 : 6, nt = pes->n_terms;
@@ -1140,8 +1130,7 @@ int MatrixPlan::upload_site_terms(const mqct_pes_t* pes) {
 int MatrixPlan::run_basis_and_pes() {
   const int threads = 256;
   const int n_beta = (int)h_beta.size();
-  const Type0Dev t0{d_ch_j2.p, d_vec2.p, d_cg.p, cg_ld, d_beta2.p, d_alpha2.p, d_gamma2.p,
-                    n_beta, n_gamma, t0_nbb, t0_naa, t0_ngg};
+  const Type0Dev t0{d_beta2.p, d_alpha2.p, d_gamma2.p, n_beta, n_gamma, t0_nbb, t0_naa, t0_ngg};
   const bool img = precision != MQCT_PREC_FP64;
   const BasisOut out{d_psi.p, d_psi32.p, tc ? tc->row_off.p : nullptr, tc ? tc->row_step.p : nullptr,
                      G2};
@@ -1390,8 +1379,6 @@ int mqct_matrix_plan_set_drain(mqct_matrix_plan* plan, int32_t slices_per_drain)
   MQCT_ARG_CHECK(p->tc, "the FP64 form has no tensor-core accumulators to drain");
   MQCT_ARG_CHECK(slices_per_drain >= 1 && slices_per_drain <= 64, "slices_per_drain %d out of 1..64",
                  slices_per_drain);
-  MQCT_ARG_CHECK(slices_per_drain == 1 || p->tc->alpha_uniform,
-                 "grouping alpha points needs equal alpha weights");
   p->tc->slices_per_drain = slices_per_drain;
   return MQCT_OK;
 }

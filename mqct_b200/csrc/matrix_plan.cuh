@@ -26,7 +26,6 @@ struct TcInfo {
   int n_parts = 1, part_c0[8] = {}, part_nc[8] = {};  // column parts of the radial axis
   int nbuf = 2;                                        // B / basis-slice buffers
   int slices_per_drain = 1;                            // alpha points per drain
-  bool alpha_uniform = true;                           // all alpha weights equal
   int pe_warps = 8;                                    // epilogue warps of the last launch
   const void* fn = nullptr;                            // kernel form of the last launch
   int pe_force = 0;                                    // 8 or 16 (tuned or set), 0: by rule
@@ -34,9 +33,8 @@ struct TcInfo {
   uint32_t b_stage = 0, psi_stage = 0;                 // bytes of one such buffer
   int n_blocks = 0, n_sm = 148;
   size_t smem = 0;
-  DevBuf<int> blk_row0, blk_n, blk_m;
+  DevBuf<int> blk_row0, blk_n;
   DevBuf<int64_t> blk_img_off;
-  DevBuf<double> walpha;
   DevBuf<unsigned long long> wmax;  // F16x3: bits of max |W| of each column
   DevBuf<int64_t> row_off;  // per basis row: its place in the image of chunk 0
   DevBuf<int> row_step;     // and the distance to its place in the next chunk
@@ -56,7 +54,7 @@ struct MatrixPlan {
   FinLaunch fin;
   double cut = 0.0;
   int pes_kind = 0, pes_n_terms = 0, pes_n_sites1 = 0, pes_n_sites2 = 0;
-  std::vector<double> Rh, h_beta, h_gamma, h_wt, h_alpha, h_walpha;
+  std::vector<double> Rh, h_beta, h_gamma, h_wt;
   // SYS_TYPE 3 runs as SYS_TYPE 4 on the parity-adapted top vectors held here
   std::vector<double> sym_top_vec;
   mqct_sys_t sym_top_sys{};
@@ -66,10 +64,10 @@ struct MatrixPlan {
   // GEMM rows: pairs grouped by m-block, each block padded to a multiple of 128
   int n_rows = 0, n_tiles = 0, n_basis_rows = 0;
   std::vector<int> h_rowa, h_rowb, h_tile_block;
-  std::vector<int> h_block_row0, h_block_n, h_block_m;  // m-blocks of the basis rows
-  DevBuf<int> d_rowa, d_rowb, d_rowm, d_k2r, d_tile_block;
+  std::vector<int> h_block_row0, h_block_n;  // m-blocks of the basis rows
+  DevBuf<int> d_rowa, d_rowb, d_k2r, d_tile_block;
   DevBuf<int> d_row_state, d_st_chan, d_st_m, d_ch_j;
-  DevBuf<double> d_vec, d_beta, d_gamma, d_wt, d_alpha, d_walpha, d_R;
+  DevBuf<double> d_vec, d_beta, d_gamma, d_wt, d_walpha, d_R;
   DevBuf<double> d_pes_p, d_pes_s1, d_pes_s2, d_pes_table;
   // SYS_TYPE 0: second rotor, Clebsch-Gordan table, the extra grid axes
   DevBuf<int> d_ch_j2;
