@@ -351,9 +351,8 @@ def run_gpu(a):
                         "inputs is reused"},
         "clocks": clk.summary(),
         # per build: rotor tables, basis, PES weights, [W column scaling (F16x3)], W image,
-        # basis image, contraction, finalize; the FP64 form: tables, basis, PES, contraction,
-        # finalize
-        "gpu_launches": int(a.steps * ((8 if prec == mq.PREC_F16X3 else 7) if tc else 5)),
+        # contraction, finalize; the FP64 form: tables, basis, PES, contraction, finalize
+        "gpu_launches": int(a.steps * ((7 if prec == mq.PREC_F16X3 else 6) if tc else 5)),
         "fp64_form": fp64,
         "accuracy": acc,
         "reference_2d_form": ref_form,
