@@ -227,7 +227,7 @@ int mqct_matrix_plan_sync(mqct_matrix_plan* plan);
  * number of split-precision products). */
 double mqct_matrix_plan_flops(const mqct_matrix_plan* plan);
 /* Split-precision plans (no counterpart in the reference): the tensor-core accumulators
- * are added to sums of two FP32 parts (48 bits) after every group of slices_per_drain alpha
+ * are added to sums of two FP32 parts (48 bits, of FP32's range) after every group of slices_per_drain alpha
  * points of a 64-point grid chunk (1..64; the plan's choice is
  * 2 on an alpha grid, else 1).  mqct_matrix_plan_layout reports that choice,
  * the number of grid-chunk ranges whose sums the finalize adds in FP64, and the number of

@@ -19,22 +19,29 @@
 // cancel.  Here an accumulator lives for one K-chunk of one group of alpha points (3 x 4 MMAs
 // of K = 16 a point) and is then added to the pair S + E by TwoSum, whose S is exact up to E:
 // against sums in FP64 a build's elements move by 1e-12 (2-norm; the FP32 partials carry 6e-8, the
-// split 5e-6), its error against 64 bits is the same 5.3e-6 (7.0e-6 with an alpha axis).  The
+// split 5e-6), its error against 64 bits is the same 5.3e-6 (7.0e-6 with an alpha axis).  E is
+// folded back into S after every chunk of several groups (48 bits); with one group a chunk it
+// grows to half an ulp of S for each of the n chunks of a unit, so that its own rounding stays below
+// n^2 2^-49 of the largest sum: 2e-12 for 36 chunks, 2e-9 for 1 000 (a fold every 16 chunks spills:
+// 612 -> 639 us).  S has FP32's range: W is scaled in F16x3; BF16x3 sums overflow at 3.4e38.  The
 // ranges of a split axis and the alpha weight (the same for every point of the midpoint grid) are
 // FP64.  The tensor-core operand of a K-chunk is the same for every alpha point of a same-m pair
 // (the e^{i m alpha} phases of the two states cancel, so the integrand at every alpha point is
 // w Re(psi_a^* psi_b) exactly), and the tensor cores contract it once per alpha point.
 //
 // What bounds it, and what the forms before measured (B200; asymmetric top + atom, j <= 8, 31 977
-// pairs, 48 x 48 points, 300 R, whole build; with the 48-point alpha axis):
+// pairs, 48 x 48 points, 300 R, whole build after a pause; builds that follow one another run at
+// 0.92 of these rates under the power cap: 5.6 ms; with the 48-point alpha axis):
 //   * FP64 instructions beside MMAs: a drain of converted values into FP64 sums and the MMAs slowed
 //     one another down to half (3 100 clocks a group of two alpha points against 1 750 for its
 //     MMAs alone; the same without the TMEM loads).  In packed FP32 adds: 7.9 -> 5.1 ms;
 //   * the operand X in shared memory was read again by every MMA, 60 clocks of shared-memory
-//     bandwidth for 56 of tensor work.  In TMEM: 5.1 -> 4.9 ms, and 64 KB of shared memory free;
+//     bandwidth for 56 of tensor work.  In TMEM: 5.1 -> 4.9 ms (4.7 of them this kernel), and 64 KB
+//     of shared memory free;
 //   * with one group a chunk (no alpha axis), forming X and the drains alternate in the same
-//     warps: 903 -> 620 us, by the cheaper drain, X through TMEM, accesses that stay in the
-//     shared address space (no spills), and sums stored as whole sectors.
+//     warps: 903 -> 612 us, by the cheaper drain, X through TMEM, accesses that stay in the
+//     shared address space (no spills in this form; 76 to 80 bytes in those of several groups), and
+//     sums stored as whole sectors.
 // The rest is the MMAs (58 to 62 clocks of N = 96 to 112 issued in order by one thread), about 300
 // clocks between two groups, and, without the alpha axis, X.
 //

@@ -23,9 +23,10 @@
 //     time, one per lane, from the path's splines.
 // tpr threads of a warp share a row, with the rows of a warp adjacent: reads of K are
 // conflict-free and the reads of bt broadcast.  Every sum has a fixed order.
-// Measured on a B200 (tables of 165 states, 1 749 elements): 400 steps of 48 trajectories 8.0 -> 2.5 ms (1.6 us a right-hand side, of
-// which the classical warp's chain and the rows' work, side by side, are 1.4), of 600 30.5 ->
-// 12.4 ms; standard batch of 48 to the end 131 -> 43 ms; AT 80 -> 20 ms with its set-up.
+// Measured on a B200 (tables of 165 states, 1 749 elements): 400 steps of 48 trajectories 8.0 ->
+// 2.5 ms (1.6 us a right-hand side, of which the classical warp's chain and the rows' work, side by
+// side, are 1.4), of 600 30.5 -> 12.4 ms; standard batches of 48 at 800 cm^-1 to the end 107 to 131
+// -> 39 to 43 ms (the longest trajectory decides); AT 80 -> 20 ms with its set-up.
 #include <algorithm>
 #include <vector>
 

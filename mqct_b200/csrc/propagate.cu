@@ -1497,9 +1497,9 @@ struct PropPlan {
   // tables fit a cluster: always with MQCT_ENGINE_RESIDENT, up to kResidentMaxBatch
   // trajectories with MQCT_ENGINE_AUTO.  It gives each trajectory a cluster of CTAs, so a
   // trajectory's steps take less time than on the per-trajectory kernel, but fewer run at
-  // once: on the 969-state asymmetric-top tables it is faster for 33 trajectories (0.64 s
-  // against 1.97 s), 512 (4.55 s against 6.04 s) and 1024 (8.9 s against 10.7 s), slower
-  // for 4096 (35.9 s against 24.2 s).  With the cluster size left to the plan, a batch that
+  // once: on the 969-state asymmetric-top tables it is faster for 33 trajectories (0.80 s
+  // against 2.72 s), 512 (4.07 s against 4.98 s) and 1024 (8.06 s against 10.8 s), slower
+  // for 4096 (32.5 s against 24.0 s).  With the cluster size left to the plan, a batch that
   // fits the clusters of eight CTAs runs on them (shorter steps), a larger one on the
   // smallest cluster that holds the tables (more clusters).
   static constexpr int64_t kResidentMaxBatch = 1024;

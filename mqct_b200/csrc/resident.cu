@@ -33,7 +33,7 @@
 // from a device queue and hands its index to the others.
 //
 // What bounds it: shared-memory wavefronts and instruction issue of the slots and the rows, one
-// after the other (about 6 us of an evaluation by four CTAs).  Before, one thread summed the
+// after the other (about 6 us an evaluation by four CTAs).  Before, one thread summed the
 // parts, took the classical stage and prepared the point between the cluster barrier and the
 // next evaluation, with four block barriers in each: 48 trajectories on the 969-state tables
 // (300 R, 700-2000 cm^-1) took 185 ms, now 170 (clusters of four; the same bits).  Keeping a
